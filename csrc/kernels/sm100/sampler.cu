@@ -7,9 +7,11 @@
 // so "a draft is accepted iff it equals the target's own sample" gives the plain sampling distribution and, with a
 // seed, the same tokens with or without speculation and at any batch size.
 //
-// Implementation: one CTA per row.  Keys are the order-preserving integer images of the logits; top-k, top-p and the
-// final inverse-CDF walk are radix descents over 8-bit digits (4 passes each) with 256-bin shared histograms of counts
-// or probability mass; ties are broken by ascending token index.  All reductions run in a fixed order.
+// Implementation: a cluster of eight CTAs per row, each with an eighth of the row in shared memory.  Keys are the
+// order-preserving integer images of the logits; top-k, top-p and the final inverse-CDF walk are radix descents over
+// 8-bit digits (4 passes each) with 256-bin histograms of counts or probability mass, summed over the cluster through
+// distributed shared memory; ties are broken by ascending token index.  Every sum is over integers, so the result does
+// not depend on how a row is cut.
 // Replaces samp_pos / samp_hist / samp_fast and accept_greedy / accept_sampled / bv_accept (m1_model.cu:476-579,
 // 1099-1452, 1536).
 #include "common.cuh"
@@ -51,15 +53,6 @@ __device__ uint32_t philox_first(unsigned long long seed, unsigned long long ctr
   return c0;
 }
 
-__device__ float block_reduce_sum(float v, float* sh) {
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float s = 0.f;
-  for (int i = 0; i < kThreads / 32; ++i) s += sh[i];
-  __syncthreads();
-  return s;
-}
 // Probability masses are fixed point (exp of a non-positive number times 2^31, so one mass fits 32 bits): integer sums
 // do not depend on the order of the additions, so every threshold of the sampler is exactly reproducible.  A histogram
 // bin is a (low, high) pair of 32-bit words: 32-bit shared-memory integer atomics are single instructions, where float
@@ -74,71 +67,120 @@ __device__ __forceinline__ void hist_add(Hist& h, uint32_t dig, unsigned long lo
   if (lo) { const uint32_t old = atomicAdd(&h.lo[dig], lo); hi += (old + lo < old) ? 1u : 0u; }
   if (hi) atomicAdd(&h.hi[dig], hi);
 }
-__device__ __forceinline__ unsigned long long hist_get(const Hist& h, int d) { return ((unsigned long long)h.hi[d] << 32) | h.lo[d]; }
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ unsigned long long block_reduce_sum_u64(unsigned long long v, unsigned long long* sh) {
-  v = warp_sum_u64(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  unsigned long long s = 0;
-  for (int i = 0; i < kThreads / 32; ++i) s += sh[i];
-  __syncthreads();
-  return s;
+constexpr int kCl = 8;                 // CTAs per row
+constexpr int kListCap = 2048;         // survivors of the filters that a CTA keeps apart
+constexpr int kCacheBytes = 160 * 1024;
+
+__device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ float block_reduce_max(float v, float* sh) {
-  v = warp_max(v);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  float s = -INFINITY;
-  for (int i = 0; i < kThreads / 32; ++i) s = fmaxf(s, sh[i]);
-  __syncthreads();
-  return s;
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {      // the same variable in CTA `rank`
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ uint32_t peer_u32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long peer_u64(uint32_t a) {
+  unsigned long long v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
 }
 
-// One pass over a row: f(value, index, valid) for every element, the same number of calls on every thread (so f may
-// use warp-wide primitives), with eight elements per thread in flight (two 16-byte loads) where the row allows it:
-// with one element per iteration a pass is bound by the latency of its loads, not by bandwidth.
+// One CTA's share of a row and the shared memory of the cluster exchange.  Exchanged variables exist twice and are used
+// in turn (`turn`): a CTA overwrites its copy only two exchanges later, after a cluster barrier that every reader of the
+// old value has passed.
+struct Share {
+  const float* x;            // values lo .. lo + n - 1 of the row, in shared memory when they fit
+  int lo, n;
+  const float* lv; const int* li; int ln;       // survivors of the filters (values, row indices) once collected; ln < 0: none
+  Hist* hist;                // [2]
+  unsigned long long* xch;   // [2]
+  unsigned long long* warp64;  // [kThreads / 32]
+  int* pick;                 // [1]
+  unsigned long long* pickv; // [2]
+  int turn;
+};
+
+// f(value, row index, valid) for every element of the share, the same number of calls on every thread of the CTA (so f
+// may use warp-wide primitives).
 template <typename F>
-__device__ __forceinline__ void scan_row(const float* x, int n, F f) {
-  const int n4 = (reinterpret_cast<uintptr_t>(x) & 15) == 0 ? n >> 2 : 0;
-  const float4* x4 = reinterpret_cast<const float4*>(x);
-  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int base = 0; base < n4; base += 2 * kThreads) {
-    const int i0 = base + (int)threadIdx.x, i1 = i0 + kThreads;
-    const bool v0 = i0 < n4, v1 = i1 < n4;
-    const float4 a = v0 ? x4[i0] : zero;
-    const float4 b = v1 ? x4[i1] : zero;
-    f(a.x, 4 * i0, v0); f(a.y, 4 * i0 + 1, v0); f(a.z, 4 * i0 + 2, v0); f(a.w, 4 * i0 + 3, v0);
-    f(b.x, 4 * i1, v1); f(b.y, 4 * i1 + 1, v1); f(b.z, 4 * i1 + 2, v1); f(b.w, 4 * i1 + 3, v1);
+__device__ __forceinline__ void scan_share(const Share& s, F f) {
+  if (s.ln >= 0) {
+    for (int base = 0; base < s.ln; base += kThreads) {
+      const int i = base + (int)threadIdx.x;
+      const bool v = i < s.ln;
+      f(v ? s.lv[i] : 0.f, v ? s.li[i] : 0, v);
+    }
+    return;
   }
-  for (int base = 4 * n4; base < n; base += kThreads) {
+#pragma unroll 4
+  for (int base = 0; base < s.n; base += kThreads) {
     const int i = base + (int)threadIdx.x;
-    f(i < n ? x[i] : 0.f, i, i < n);
+    const bool v = i < s.n;
+    f(v ? s.x[i] : 0.f, s.lo + i, v);
   }
+}
+
+enum ClOp { CL_SUM, CL_MAXF, CL_MIN };
+// Reduction of one 64-bit value per thread over the CTA and the cluster; every thread gets the result.
+template <ClOp OP>
+__device__ unsigned long long cluster_reduce(Share& s, unsigned long long v) {
+  auto comb = [](unsigned long long a, unsigned long long b) -> unsigned long long {
+    if (OP == CL_SUM) return a + b;
+    if (OP == CL_MIN) return a < b ? a : b;
+    return (unsigned long long)__float_as_uint(fmaxf(__uint_as_float((uint32_t)a), __uint_as_float((uint32_t)b)));
+  };
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = comb(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) s.warp64[threadIdx.x >> 5] = v;
+  __syncthreads();
+  const int t = s.turn;
+  s.turn ^= 1;
+  if (threadIdx.x < 32) {
+    v = s.warp64[threadIdx.x];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = comb(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if (threadIdx.x == 0) s.xch[t] = v;
+  }
+  cluster_sync();
+  v = peer_u64(peer_addr(&s.xch[t], 0));
+#pragma unroll
+  for (uint32_t r = 1; r < kCl; ++r) v = comb(v, peer_u64(peer_addr(&s.xch[t], r)));
+  return v;
 }
 
 // Radix descent: finds the largest key prefix such that the mass of all elements with a strictly larger key is
-// <= target (mass = probability or count).  On return *above = mass strictly above the final key, *at = mass of
-// elements equal to the final key.  `keep_min`: elements with key < keep_min are ignored.
+// <= target (mass = probability or count).  On return *above = mass strictly above the final key.
+// `keep_min`: elements with key < keep_min are ignored.
 template <bool COUNT>
-__device__ uint32_t radix_descend(const float* x, int n, float mx, float inv_t, uint32_t keep_min, unsigned long long target,
-                                  Hist& hist, unsigned long long* above_out, unsigned long long* at_out) {
+__device__ uint32_t radix_descend(Share& s, float mx, float inv_t, uint32_t keep_min, unsigned long long target,
+                                  unsigned long long* above_out) {
   uint32_t prefix = 0, mask = 0;
-  unsigned long long above = 0, at = 0;
+  unsigned long long above = 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int shift = 24; shift >= 0; shift -= 8) {
-    for (int i = threadIdx.x; i < 256; i += kThreads) { hist.lo[i] = 0; hist.hi[i] = 0; }
+    const int t = s.turn;
+    s.turn ^= 1;
+    Hist& hist = s.hist[t];
+    if (threadIdx.x < 256) { hist.lo[threadIdx.x] = 0; hist.hi[threadIdx.x] = 0; }
     __syncthreads();
     // Logits crowd into a few digits at the upper levels, where one shared-memory atomic per element would serialise
     // the warp: lanes that share a digit with at least seven others are summed in registers first and their leader
     // adds once; the rest add for themselves.
-    const int lane = threadIdx.x & 31;
-    scan_row(x, n, [&](float xv, int, bool valid) {
+    scan_share(s, [&](float xv, int, bool valid) {
       const uint32_t k = key_of(xv);
       const bool on = valid && k >= keep_min && (k & mask) == prefix;
+      if (!__any_sync(0xffffffffu, on)) return;
       const uint32_t dig = on ? (k >> shift) & 255u : 0xFFFFFFFFu;
       const unsigned long long v = !on ? 0ull : (COUNT ? 1ull : mass_of(xv, mx, inv_t));
       const unsigned peers = __match_any_sync(0xffffffffu, dig);
@@ -153,19 +195,42 @@ __device__ uint32_t radix_descend(const float* x, int n, float mx, float inv_t, 
       }
       if (on && !big) hist_add(hist, dig, v);
     });
+    cluster_sync();
+    // the row's digit d, walked from high to low, is the first with above + mass(digits >= d) > target (0 if none):
+    // thread i < 256 takes digit 255 - i, so the running masses are prefix sums over the threads
+    unsigned long long h = 0, inc = 0;
+    if (threadIdx.x < 256) {
+      const int d = 255 - (int)threadIdx.x;
+#pragma unroll
+      for (uint32_t r = 0; r < kCl; ++r) {
+        const uint32_t lo = peer_u32(peer_addr(&hist.lo[d], r)), hi = peer_u32(peer_addr(&hist.hi[d], r));
+        h += ((unsigned long long)hi << 32) | lo;
+      }
+      inc = h;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long p = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += p;
+      }
+      if (lane == 31) s.warp64[warp] = inc;
+    }
+    if (threadIdx.x == 0) *s.pick = 255;
     __syncthreads();
-    // walk digits from high to low until the running mass passes the target (every thread does the same walk)
-    int d = 255;
-    unsigned long long run = above;
-    for (; d > 0; --d) { const unsigned long long hd = hist_get(hist, d); if (run + hd > target) break; run += hd; }
-    above = run;
-    at = hist_get(hist, d);
-    prefix |= (uint32_t)d << shift;
+    if (threadIdx.x < 256) {
+      inc += above;
+      for (int w = 0; w < warp; ++w) inc += s.warp64[w];
+      const bool past = inc > target;
+      if (past && threadIdx.x < 255) atomicMin(s.pick, (int)threadIdx.x);
+    }
+    __syncthreads();
+    const int pick = *s.pick;
+    if ((int)threadIdx.x == pick) s.pickv[t] = inc - h;
+    __syncthreads();
+    above = s.pickv[t];
+    prefix |= (uint32_t)(255 - pick) << shift;
     mask |= 255u << shift;
-    __syncthreads();
   }
   *above_out = above;
-  *at_out = at;
   return prefix;
 }
 
@@ -173,30 +238,60 @@ __device__ uint32_t radix_descend(const float* x, int n, float mx, float inv_t, 
 
 // Determinism: counts and fixed-point masses are integers, so every histogram, threshold and the final walk are
 // independent of the order in which threads add; equal keys are ordered by token index.
-__global__ void __launch_bounds__(kThreads) sample_rows_kernel(const SampleArgs a) {
-  __shared__ float sh[kThreads / 32];
-  __shared__ unsigned long long sh64[kThreads / 32];
-  __shared__ Hist hist;
+//
+// What bounds it: about fifteen passes over the row.  With one CTA per row (the earlier kernel) a pass moved 600 KB of
+// logits from L2 through a single SM and walked its 256 bins serially on every thread: 518 us for 16 rows of 151936
+// logits.  Here a row is read from memory once, a pass costs 19 values per thread plus a cluster barrier, and passes
+// after top-k or min-p touch the survivors only: 93 us.
+__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_rows_kernel(const SampleArgs a, int share, int cached) {
+  extern __shared__ __align__(16) float cache[];
+  __shared__ Hist hist[2];
+  __shared__ unsigned long long xch[2], warp64[kThreads / 32], pickv[2];
+  __shared__ float list_v[kListCap];
+  __shared__ int list_i[kListCap];
+  __shared__ int s_pick, s_list;
   pdl_wait();
   pdl_launch_dependents();
-  const int row = blockIdx.x;
-  const float* x = a.logits + (size_t)row * a.ld;
-  const int n = a.vocab;
+  const int row = blockIdx.x / kCl;
+  const int rank = (int)cluster_rank();
+  Share s;
+  s.lo = min(rank * share, a.vocab);
+  s.n = min(share, a.vocab - s.lo);
+  s.ln = -1; s.lv = list_v; s.li = list_i;
+  s.hist = hist; s.xch = xch; s.warp64 = warp64; s.pick = &s_pick; s.pickv = pickv;
+  s.turn = 0;
+  const float* gx = a.logits + (size_t)row * a.ld + s.lo;
+  s.x = gx;
   float mx = -INFINITY;
-  scan_row(x, n, [&](float xv, int, bool valid) { if (valid) mx = fmaxf(mx, xv); });
-  mx = block_reduce_max(mx, sh);
+  if (cached) {
+    int i0 = 0;
+    if ((reinterpret_cast<uintptr_t>(gx) & 15) == 0) {
+      const int n4 = s.n >> 2;
+#pragma unroll 4
+      for (int i = threadIdx.x; i < n4; i += kThreads) {
+        const float4 v = reinterpret_cast<const float4*>(gx)[i];
+        reinterpret_cast<float4*>(cache)[i] = v;
+        mx = fmaxf(fmaxf(mx, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
+      }
+      i0 = 4 * n4;
+    }
+    for (int i = i0 + threadIdx.x; i < s.n; i += kThreads) { const float v = gx[i]; cache[i] = v; mx = fmaxf(mx, v); }
+    s.x = cache;
+  } else {
+    for (int i = threadIdx.x; i < s.n; i += kThreads) mx = fmaxf(mx, gx[i]);
+  }
+  mx = __uint_as_float((uint32_t)cluster_reduce<CL_MAXF>(s, __float_as_uint(mx)));     // its barriers also publish `cache` to the CTA
   const float T = a.temperature ? a.temperature[row] : 0.f;
   const int topk = a.top_k ? a.top_k[row] : 0;
-  if (T <= 0.f || topk == 1) {
-    // greedy: lowest index among the maxima
-    int best = 0x7fffffff;
-    scan_row(x, n, [&](float xv, int i, bool valid) { if (valid && xv == mx) best = min(best, i); });
-    __shared__ int sbest[kThreads / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if ((threadIdx.x & 31) == 0) sbest[threadIdx.x >> 5] = best;
-    __syncthreads();
-    if (threadIdx.x == 0) { int b = sbest[0]; for (int i = 1; i < kThreads / 32; ++i) b = min(b, sbest[i]); a.out[row] = b; }
+  auto lowest_max = [&]() {          // lowest index among the maxima
+    unsigned long long best = 0x7fffffffull;
+    scan_share(s, [&](float xv, int i, bool valid) { if (valid && xv == mx) best = min(best, (unsigned long long)i); });
+    best = cluster_reduce<CL_MIN>(s, best);
+    if (rank == 0 && threadIdx.x == 0) a.out[row] = (int)best;
+  };
+  if (T <= 0.f || topk == 1) {       // greedy
+    lowest_max();
+    cluster_sync();                  // no CTA leaves while another still reads its shared memory
     return;
   }
   const float inv_t = 1.f / T;
@@ -205,62 +300,70 @@ __global__ void __launch_bounds__(kThreads) sample_rows_kernel(const SampleArgs 
   const float minp = a.min_p ? a.min_p[row] : 0.f;
   if (minp > 0.f) keep_min = max(keep_min, key_of(mx + T * __logf(minp)));
   // top-k: key of the k-th largest logit (ties at the threshold are all kept; the index rule orders them)
-  if (topk > 1 && topk < n) {
-    unsigned long long above, at;
-    const uint32_t kth = radix_descend<true>(x, n, mx, inv_t, 0u, (unsigned long long)(topk - 1), hist, &above, &at);
+  if (topk > 1 && topk < a.vocab) {
+    unsigned long long above;
+    const uint32_t kth = radix_descend<true>(s, mx, inv_t, 0u, (unsigned long long)(topk - 1), &above);
     keep_min = max(keep_min, kth);
   }
+  if (keep_min > 0) {                // later passes read this CTA's survivors only, if there is room for them
+    if (threadIdx.x == 0) s_list = 0;
+    __syncthreads();
+    scan_share(s, [&](float xv, int i, bool valid) {
+      if (valid && key_of(xv) >= keep_min) {
+        const int at = atomicAdd(&s_list, 1);
+        if (at < kListCap) { list_v[at] = xv; list_i[at] = i; }
+      }
+    });
+    __syncthreads();
+    if (s_list <= kListCap) s.ln = s_list;
+  }
+  auto mass_left = [&]() {           // mass of what is left
+    unsigned long long z = 0;
+    scan_share(s, [&](float xv, int, bool valid) { if (valid && key_of(xv) >= keep_min) z += mass_of(xv, mx, inv_t); });
+    return cluster_reduce<CL_SUM>(s, z);
+  };
   // top-p over what is left: smallest descending prefix whose mass reaches top_p * Z
   const float topp = a.top_p ? a.top_p[row] : 1.f;
   if (topp < 1.f) {
-    unsigned long long z = 0;
-    scan_row(x, n, [&](float xv, int, bool valid) { if (valid && key_of(xv) >= keep_min) z += mass_of(xv, mx, inv_t); });
-    z = block_reduce_sum_u64(z, sh64);
-    unsigned long long above, at;
-    const uint32_t cut = radix_descend<false>(x, n, mx, inv_t, keep_min, (unsigned long long)((double)topp * (double)z), hist, &above, &at);
+    const unsigned long long z = mass_left();
+    unsigned long long above;
+    const uint32_t cut = radix_descend<false>(s, mx, inv_t, keep_min, (unsigned long long)((double)topp * (double)z), &above);
     keep_min = max(keep_min, cut);
   }
   // draw
-  unsigned long long z = 0;
-  scan_row(x, n, [&](float xv, int, bool valid) { if (valid && key_of(xv) >= keep_min) z += mass_of(xv, mx, inv_t); });
-  z = block_reduce_sum_u64(z, sh64);                         // at least 2^31: the maximum always survives the filters
+  const unsigned long long z = mass_left();                  // at least 2^31: the maximum always survives the filters
   const uint32_t r = philox_first(a.seed ? a.seed[row] : 0ull, (unsigned long long)(a.position ? a.position[row] : 0));
   const double u = ((double)(r >> 8) + 0.5) * (1.0 / 16777216.0);
   unsigned long long target = (unsigned long long)(u * (double)z);
   if (z > 0 && target >= z) target = z - 1;
-  unsigned long long above, at;
-  const uint32_t key = radix_descend<false>(x, n, mx, inv_t, keep_min, target, hist, &above, &at);
+  unsigned long long above;
+  const uint32_t key = radix_descend<false>(s, mx, inv_t, keep_min, target, &above);
   // among the tokens that share the final key, walk by ascending index: the `want`-th of them wins
   const unsigned long long w = mass_of(__uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), mx, inv_t);
   const unsigned long long rank64 = w > 0 && target > above ? (target - above) / w : 0ull;
-  const int rank = (int)(rank64 > 1000000000ull ? 1000000000ull : rank64);
-  float cnt = 0.f;
-  scan_row(x, n, [&](float xv, int, bool valid) { cnt += valid && key_of(xv) == key ? 1.f : 0.f; });
-  cnt = block_reduce_sum(cnt, sh);                          // exact: integers below 2^24
-  const int want = min(rank, max((int)cnt - 1, 0));
-  if ((int)cnt == 0) {                                       // rounding pushed the walk past the last bin: take the mode
-    __shared__ int s_fb;
-    if (threadIdx.x == 0) s_fb = 0x7fffffff;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kThreads) if (x[i] == mx) atomicMin(&s_fb, i);
-    __syncthreads();
-    if (threadIdx.x == 0) a.out[row] = s_fb;
-    return;
+  const int nth = (int)(rank64 > 1000000000ull ? 1000000000ull : rank64);
+  unsigned long long same = 0;
+  scan_share(s, [&](float xv, int, bool valid) { same += valid && key_of(xv) == key ? 1u : 0u; });
+  const int cnt = (int)cluster_reduce<CL_SUM>(s, same);
+  if (cnt == 0) {                                            // rounding pushed the walk past the last bin: take the mode
+    s.ln = -1;
+    lowest_max();
+  } else if (cnt == 1) {                                     // the usual case: one token owns the key
+    scan_share(s, [&](float xv, int i, bool valid) { if (valid && key_of(xv) == key) a.out[row] = i; });
+  } else {
+    // smallest index I with (number of equal-key tokens at index <= I) == want + 1, by bisection over the index range
+    const int want = min(nth, cnt - 1);
+    int lo = 0, hi = a.vocab - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      unsigned long long c = 0;
+      scan_share(s, [&](float xv, int i, bool valid) { c += valid && i <= mid && key_of(xv) == key ? 1u : 0u; });
+      c = cluster_reduce<CL_SUM>(s, c);
+      if ((int)c >= want + 1) hi = mid; else lo = mid + 1;
+    }
+    if (rank == 0 && threadIdx.x == 0) a.out[row] = lo;
   }
-  if ((int)cnt == 1) {                                       // the usual case: one token owns the key
-    scan_row(x, n, [&](float xv, int i, bool valid) { if (valid && key_of(xv) == key) a.out[row] = i; });
-    return;
-  }
-  // smallest index I with (number of equal-key tokens at index <= I) == want + 1, by bisection over the index range
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    float c = 0.f;
-    for (int i = threadIdx.x; i <= mid; i += kThreads) c += key_of(x[i]) == key ? 1.f : 0.f;
-    c = block_reduce_sum(c, sh);
-    if ((int)c >= want + 1) hi = mid; else lo = mid + 1;
-  }
-  if (threadIdx.x == 0) a.out[row] = lo;
+  cluster_sync();
 }
 
 // Longest-prefix acceptance for one or more verify blocks.  Block b covers rows [row0[b], row0[b] + cnt[b]): row 0 is
@@ -285,13 +388,17 @@ using namespace b2;
 
 B2_API int b2_sample_rows(const SampleArgs* a, int rows, cudaStream_t st) {
   if (!a || rows <= 0 || a->vocab <= 0 || !a->logits || !a->out) return B2_ERR_ARG;
+  const int share = ((a->vocab + kCl - 1) / kCl + 3) & ~3;             // multiple of four: shares keep the row's alignment
+  const int cached = (long)share * 4 <= kCacheBytes;
+  if (cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCacheBytes) != cudaSuccess) return B2_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(rows); cfg.blockDim = dim3(kThreads); cfg.stream = st;
+  cfg.gridDim = dim3((unsigned)rows * kCl); cfg.blockDim = dim3(kThreads); cfg.stream = st;
+  cfg.dynamicSmemBytes = cached ? (size_t)share * 4 : 0;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, sample_rows_kernel, *a) == cudaSuccess ? B2_OK : B2_ERR_LAUNCH;
+  return cudaLaunchKernelEx(&cfg, sample_rows_kernel, *a, share, cached) == cudaSuccess ? B2_OK : B2_ERR_LAUNCH;
 }
 
 B2_API int b2_spec_accept(const int* ids, const int* target, const int* row0, const int* cnt, int n_blocks, int* n_emitted,
