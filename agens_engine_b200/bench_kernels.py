@@ -237,7 +237,7 @@ def bench_mm(args):
                     L.mm(ln, x, ws, out=out)
 
             med, best = graph_time_us(launch_all, len(lins))
-            print(json.dumps(dict(name=name, n=n, k=k, bits=bits, m=args.m, ks=lib.b2_wq_mm_ks(n, k), us=round(med, 1),
+            print(json.dumps(dict(name=name, n=n, k=k, bits=bits, m=args.m, ctas=lib.b2_wq_mm_ctas(n, k), us=round(med, 1),
                                   gbs=round(nb / med / 1e3, 0), frac_hbm=round(nb / med / 1e3 / pk["hbm_gbs"], 3),
                                   tflops=round(2.0 * args.m * n * k / med / 1e6, 1))), flush=True)
     print(json.dumps({"peaks": pk, "timing": "CUDA graph of back-to-back launches (activation prologue + GEMM) over rotating weight "
