@@ -271,19 +271,22 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
     if resid is not None:
         a.resid, a.ldr = ptr(resid), resid.stride(0)
     a.ss_out = ptr(ss_out)
-    a.vworkers = lib.b2_wq_gemv_vworkers(lin.n, lin.k, lin.ks, a.rb)
-    a.fmax = lib.b2_wq_gemv_fmax(lin.n, lin.k, lin.ks, a.rb)
-    need = lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, a.rb, m)
-    if need > ws.scratch.numel() or lin.n_panels() > ws.counters.numel():
-        raise RuntimeError(f"GEMV workspace too small: need {need} floats, {lin.n_panels()} counters")
     a.scratch, a.counters = ptr(ws.scratch), ptr(ws.counters)
     a.status = ptr(ws.status)
-    a.debug = GEMV_DEBUG
-    a.trace = ptr(TRACE_BUFFER)
-    if tp is not None:
-        a.tp = tp
+    if tp is None:
+        need = lib.b2_wq_gemv8_scratch_floats(lin.n, lin.k, m)
+    else:
+        a.vworkers = lib.b2_wq_gemv_vworkers(lin.n, lin.k, lin.ks, a.rb)
+        a.fmax = lib.b2_wq_gemv_fmax(lin.n, lin.k, lin.ks, a.rb)
+        a.debug, a.trace, a.tp = GEMV_DEBUG, ptr(TRACE_BUFFER), tp
+        need = lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, a.rb, m)
+    if need > ws.scratch.numel() or lin.n_panels() > ws.counters.numel():
+        raise RuntimeError(f"GEMV workspace too small: need {need} floats, {lin.n_panels()} counters")
     with torch.cuda.device(dev):
-        check(lib.b2_wq_gemv(C.byref(a), current_stream()), "b2_wq_gemv")
+        if tp is None:
+            check(lib.b2_wq_gemv8(C.byref(a), current_stream()), "b2_wq_gemv8")
+        else:                                   # the push all-reduce epilogue is in the other kernel of the family
+            check(lib.b2_wq_gemv(C.byref(a), current_stream()), "b2_wq_gemv")
     return out
 
 

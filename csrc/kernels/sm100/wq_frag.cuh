@@ -51,12 +51,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after about two seconds and reports failure instead of hanging the GPU.
+// Bounded wait: gives up after about two seconds and reports failure instead of hanging the GPU.  The clock is looked at
+// on every 256th try only: reading it takes longer than a try.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait(bar, parity)) {
-    if (globaltimer_ns() - t0 > 2000000000ull) return false;
+  uint64_t t0 = 0;
+  for (unsigned it = 1; !mbar_try_wait(bar, parity); ++it) {
+    if ((it & 255u) == 0u) {
+      const uint64_t t = globaltimer_ns();
+      if (!t0) t0 = t;
+      else if (t - t0 > 2000000000ull) return false;
+    }
   }
   return true;
 }

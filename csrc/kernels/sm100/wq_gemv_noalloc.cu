@@ -87,7 +87,8 @@ extern "C" int b2_wq_gemv_noalloc(const uint8_t* wq, int n, int k, int bits, int
   a.scratch = s->partials;
   a.counters = s->counters;
   a.status = s->status;
-  const int st = b2_wq_gemv(&a, stream);
+  // the kernel of the regular entry point, unless its scratch exceeds the array where the other's does not
+  const int st = b2_wq_gemv8_scratch_floats(n, k, m) <= (long)B2_NOALLOC_SCRATCH_FLOATS ? b2_wq_gemv8(&a, stream) : b2_wq_gemv(&a, stream);
   if (st != 0) {
     set_err(err, st == 1 ? "b2_wq_gemv_noalloc: the GEMV launcher rejected the arguments (alignment of x / ldx?)"
                          : "b2_wq_gemv_noalloc: kernel launch failed");

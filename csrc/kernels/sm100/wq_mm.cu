@@ -60,23 +60,10 @@ constexpr int kTmemColsM = 512;
 __device__ __forceinline__ void mbar_arrive_m(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait (about two seconds).  The clock is looked at on every 256th try only.
-__device__ __forceinline__ bool mbar_wait_m(uint32_t bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
-  uint64_t t0 = 0;
-  for (unsigned it = 1; !mbar_try_wait(bar, parity); ++it) {
-    if ((it & 255u) == 0u) {
-      const uint64_t t = globaltimer_ns();
-      if (!t0) t0 = t;
-      else if (t - t0 > 2000000000ull) return false;
-    }
-  }
-  return true;
-}
-// The same by a whole warp: its lanes may leave the wait at different tries, and the tcgen05.ld and .st that follow are
+// mbar_wait_bounded by a whole warp: its lanes may leave the wait at different tries, and the tcgen05.ld and .st that follow are
 // .aligned; the vote brings the lanes back together and makes the answer uniform.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait_m(bar, parity)) != 0;
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)) != 0;
 }
 __device__ __forceinline__ void tma_load_2d_m(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -263,7 +250,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       int tile = tile0, kb = kb0;
       RingPos r;
       for (int i = 0; i < nu; ++i, r.next(RS)) {
-        if (i >= RS && !mbar_wait_m(smem_u32(&raw_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
+        if (i >= RS && !mbar_wait_bounded(smem_u32(&raw_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
         const uint32_t bar = smem_u32(&raw_full[r.s]);
         mbar_expect_tx(bar, (uint32_t)RAW);
 #pragma unroll
@@ -282,7 +269,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       int kb = kb0;
       RingPos r;
       for (int i = 0; i < nu; ++i, r.next(NB)) {
-        if (i >= NB && !mbar_wait_m(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
+        if (i >= NB && !mbar_wait_bounded(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
         const uint32_t bar = smem_u32(&op_full[r.s]);
         mbar_expect_tx(bar, 2 * x_sub);
         tma_load_2d_m(x_ring + 2 * r.s * x_sub, &map_x, kb * 128, 0, bar);
@@ -300,8 +287,8 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       const uint32_t dx_step = (2 * x_sub) >> 4, dx_half = x_sub >> 4;
       for (int i = 0; i < nu; ++i, r.next(NB)) {
         const bool first = i == 0 || kb == 0, last = i == nu - 1 || kb == nbat - 1;
-        if (first && frag >= nd && !mbar_wait_m(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
-        if (!mbar_wait_m(smem_u32(&op_full[r.s]), r.ph)) { atomicExch(&s_failed, 1); break; }
+        if (first && frag >= nd && !mbar_wait_bounded(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
+        if (!mbar_wait_bounded(smem_u32(&op_full[r.s]), r.ph)) { atomicExch(&s_failed, 1); break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint64_t dx = dx_base + (uint32_t)r.s * dx_step;
         const uint32_t ta = tmem_base + (uint32_t)(r.s * 64), td = tmem_d0 + (uint32_t)(d.s * a.n_pad);

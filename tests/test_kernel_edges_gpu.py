@@ -48,3 +48,23 @@ def test_dequant_blocks(bits, group, offset):
     rc = _lib.cuda_lib().b2_wq_dequant(buf.data_ptr() + offset, n, k, bits, group, out.data_ptr(), ldo, _lib.current_stream())
     assert rc == 0
     assert torch.equal(out[:, :k].cpu(), ql.dequant().to(torch.bfloat16)) and bool((out[:, k:] == 7.0).all())
+
+
+# one unit, one panel, k in two and more slices (above 5120 inputs), panels shared by CTAs, panels cut between CTAs
+@pytest.mark.parametrize("n,k", [(32, 128), (160, 1024), (96, 5248), (64, 25600), (37888, 128)])
+@pytest.mark.parametrize("bits,group", [(2, 64), (3, 128), (4, 128)])
+def test_gemv_work_split(n, k, bits, group):
+    """Every row count gives the same bits, and they agree with fp64 within the fp16 activations that carry 1 / c
+    (three roundings of 2^-11 on inputs of random sign: below 1e-3 of the result's norm)."""
+    lin = L.WqLinear.random(n, k, bits, group, DEV, seed=7)
+    torch.cuda.synchronize()
+    ws = L.GemvWorkspace(DEV)
+    ws.mm_min_rows = 33
+    torch.manual_seed(3)
+    x = torch.randn(19, k, device=DEV).to(torch.bfloat16)
+    ref = x.double() @ lin.dequant_cpu().double().to(DEV).t()
+    y = L.gemv(lin, x, ws, epi=_lib.EPI_F32)
+    assert (y.double() - ref).norm() < 1e-3 * ref.norm()
+    for m in (1, 2, 7, 8, 9):
+        assert torch.equal(L.gemv(lin, x[:m], ws, epi=_lib.EPI_F32), y[:m]), m
+    assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
