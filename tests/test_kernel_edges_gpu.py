@@ -68,3 +68,34 @@ def test_gemv_work_split(n, k, bits, group):
     for m in (1, 2, 7, 8, 9):
         assert torch.equal(L.gemv(lin, x[:m], ws, epi=_lib.EPI_F32), y[:m]), m
     assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
+
+
+# 128-row tiles, two per CTA, blocks of 128 keys: chunks that leave the second tile empty or ragged, contexts at and around
+# a block's end, one to 128 query heads per KV head, scores that keep growing (the reference maximum moves several times)
+@pytest.mark.parametrize("T,pos0,hq,hkv,grow", [(1, 0, 8, 8, 0), (64, 63, 16, 8, 0), (64, 64, 16, 8, 0), (65, 64, 64, 8, 0), (300, 511, 8, 1, 0),
+                                                (130, 700, 16, 8, 1), (3, 250, 128, 1, 1)])
+def test_prefill_attention_tiles(T, pos0, hq, hkv, grow):
+    """Against fp64; P is bf16 (relative 2^-9 per term, random), the result is rounded to bf16: below 6e-3 of the norm.
+    Slots of the pool that the sequence does not use hold NaN."""
+    torch.manual_seed(T + pos0)
+    n = pos0 + T
+    npg = (n + 15) // 16
+    k, v = torch.randn(n, hkv, 128, device=DEV).to(torch.bfloat16), torch.randn(n, hkv, 128, device=DEV).to(torch.bfloat16)
+    q = torch.randn(T, hq, 128, device=DEV).to(torch.bfloat16)
+    if grow:
+        k[:, :, 0] += torch.arange(n, device=DEV).to(torch.bfloat16)[:, None] / 20
+        q[:, :, 0] = 20.0
+    pool = torch.full((npg + 2, 2, hkv, 16, 128), float("nan"), dtype=torch.bfloat16, device=DEV)
+    perm = torch.randperm(npg + 2)[:npg]
+    for i in range(npg):
+        c = min(16, n - 16 * i)
+        pool[perm[i], 0, :, :c] = k[16 * i:16 * i + c].transpose(0, 1)
+        pool[perm[i], 1, :, :c] = v[16 * i:16 * i + c].transpose(0, 1)
+    from agens_engine_b200.ops import attention as A
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = A.attn_prefill_tc(q.reshape(T, -1).contiguous(), pool, perm.to(torch.int32)[None].to(DEV), 0, pos0, hq, hkv, status=status)
+    s = torch.einsum("thd,lhd->htl", q.double(), k.double().repeat_interleave(hq // hkv, 1)) / 128 ** 0.5
+    s = s.masked_fill(torch.arange(n, device=DEV)[None, None] > (pos0 + torch.arange(T, device=DEV))[None, :, None], float("-inf"))
+    ref = torch.einsum("htl,lhd->thd", torch.softmax(s, -1), v.double().repeat_interleave(hq // hkv, 1)).reshape(T, -1)
+    assert int(status.item()) == 0
+    assert (out.double() - ref).norm() < 6e-3 * ref.norm()
