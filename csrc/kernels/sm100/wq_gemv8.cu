@@ -2,33 +2,35 @@
 // chunks of eight.  Same weight layout, arithmetic per group and epilogues as wq_gemv.cu, whose kernel stays for the
 // tensor-parallel push epilogue.
 //
-// Work: the units (32-row panel, 128-k batch) of the matrix, listed slice by slice of k (one slice up to 5120 inputs,
-// else slices of at most 2560, so that the activations a CTA needs fit its shared memory), panel by panel, batch by
-// batch.  CTA c takes the c-th share of the list, its sixteen warps consecutive shares of that.  A panel segment inside
-// one warp is finished by that warp; one that several warps share meets in shared memory, one that several CTAs share in
-// scratch memory, where the last arriver adds the parts in list order.  Matrices with at least eight panels per CTA are
-// cut at panels and need no scratch.  Cuts and orders depend on (n, k) only, so a row's bits do not depend on the rows
-// that travel with it.
+// Work: the units (32-row panel, 128-k batch) of the matrix.  k is cut into equal slices of at most 5120 inputs, so that
+// a CTA's activations fit its shared memory at eight rows, and every slice has the same number of CTAs; CTA c of a slice
+// takes the c-th share of the slice's units in panel order, its sixteen warps consecutive shares of that.  A panel
+// segment inside one warp is finished by that warp; one that several warps share meets in shared memory, one that several
+// CTAs or slices share in scratch memory, where the last arriver adds the parts in (slice, CTA) order.  Matrices of one
+// slice with at least eight panels per CTA are cut at panels and need no scratch.  Cuts and orders depend on (n, k) only,
+// so a row's bits do not depend on the rows that travel with it.
 //
-// One CTA of 16 warps per SM at 64 registers and, for one or two rows, under half of the shared memory: the next linear
-// of a captured step becomes resident while this one runs and fills its weight rings before its dependency wait, so the
-// launch, the first DRAM round trip and the tail of the kernel before overlap.
+// One CTA of 16 warps per SM at full registers.  (64 registers and half of the shared memory, so that the next linear's
+// CTAs could prefetch beside this one, measured slower: 747 against 471 us for four 32B layers and the head at one row --
+// the early CTAs keep the attention kernels between the linears off the SMs.)
 //
-// What bounds it: large matrices the inner loop (256 warp instructions a unit, the logic pipe at half rate: some 420 cycles
-// per scheduler against 380 of DRAM time for 4 bits), small ones the hand-over.  The kernel of wq_gemv.cu staged every
-// row of a CTA's slice and summed every row's parts one after the other, and kept two CTAs of eight warps whose shared
-// memory left one CTA from five rows on.  4 bits, graph replays over weights larger than L2, before -> now: one row
-// gate_up 36 -> 32 us, lm_head 82 -> 81, down 25 -> 26, qkv 14.0 -> 14.0, 4096 x 1024 7.2 -> 4.3; eight rows gate_up
-// 101 -> 39, lm_head 199 -> 90, down 191 -> 33, qkv 64 -> 19, o 79 -> 16.
+// What bounds it: large matrices the inner loop (the logic pipe takes two cycles an instruction and scheduler, some 110 of
+// them a unit, and 16 half-precision MMAs of 8) and, at 4 bits, DRAM; small ones the fixed 4 us of launch, staging and
+// hand-over.  The kernel of wq_gemv.cu staged every row of a CTA's slice and summed every row's parts one after the
+// other, and its shared memory left one CTA of eight warps per SM from five rows on.  4 bits, graph replays over weights
+// larger than L2, before -> now: one row gate_up 36 -> 27 us, lm_head 82 -> 68 (floor 63), down 25 -> 18, qkv 14.0 ->
+// 11.4, o 13.6 -> 10.6, 4096 x 1024 7.2 -> 3.8; eight rows gate_up 101 -> 34, lm_head 199 -> 76, down 191 -> 25, qkv
+// 64 -> 16, o 79 -> 15.
 #include "wq_frag.cuh"
 #include "wq_gemv.cuh"
 
 namespace b2 {
 
 struct Gemv8Plan {
-  int ctas, slices, panel_cut;   // functions of (n, k)
+  int slices, per_slice;         // functions of (n, k): slices of k, CTAs per slice
+  int panel_cut;
   int fmax;                      // most CTAs that share a segment
-  int xb;                        // batches of activations a CTA stages
+  int xb;                        // batches of the longest slice
   int nst;                       // ring stages per warp
 };
 
@@ -36,42 +38,13 @@ namespace {
 
 constexpr int kW8 = 16, kT8 = kW8 * 32;
 
-// Position in the unit list.
-struct Cur {
-  int s, len, base;              // slice, its batches, its first batch
-  int pan, b;
-};
 __device__ __forceinline__ int slice_base(int s, int nbat, int S) { return s * nbat / S; }
-__device__ __forceinline__ Cur cur_at(unsigned u, int npan, int nbat, int S) {
-  Cur c;
-  c.s = 0;
-  if (S > 1) {
-    while (c.s + 1 < S && (unsigned)npan * (unsigned)slice_base(c.s + 1, nbat, S) <= u) ++c.s;
-  }
-  c.base = slice_base(c.s, nbat, S);
-  c.len = slice_base(c.s + 1, nbat, S) - c.base;
-  const unsigned r = u - (unsigned)npan * (unsigned)c.base;
-  c.pan = (int)(r / (unsigned)c.len);
-  c.b = (int)(r - (unsigned)c.pan * (unsigned)c.len);
-  return c;
-}
-__device__ __forceinline__ void cur_next(Cur& c, int npan, int nbat, int S) {
-  if (++c.b == c.len) {
-    c.b = 0;
-    if (++c.pan == npan) {
-      c.pan = 0;
-      ++c.s;
-      c.base = slice_base(c.s, nbat, S);
-      c.len = slice_base(c.s + 1, nbat, S) - c.base;
-    }
-  }
-}
 
 }  // namespace
 
 // ONE: a single row (columns other than the token's are not scaled); otherwise two to eight rows.
 template <int BITS, int GROUP, bool ONE>
-__global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, const Gemv8Plan p) {
+__global__ void __launch_bounds__(kT8, 1) wq_gemv8_kernel(const WqGemvArgs a, const Gemv8Plan p) {
   constexpr int GPB = 128 / GROUP;
   constexpr int MP = ONE ? 1 : 8;
   using R = Ring<BITS, GROUP, 2>;
@@ -79,8 +52,12 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int m = ONE ? 1 : a.m;
-  const int npan = a.n >> 5, nbat = a.k >> 7, S = p.slices, G = p.ctas;
-  const unsigned U = (unsigned)npan * (unsigned)nbat;
+  const int npan = a.n >> 5, nbat = a.k >> 7, S = p.slices;
+  const unsigned G = (unsigned)p.per_slice;
+  const int slice = (int)(blockIdx.x / G);
+  const unsigned cta = blockIdx.x - (unsigned)slice * G;
+  const int base = slice_base(slice, nbat, S), len = slice_base(slice + 1, nbat, S) - base;   // batches of this slice
+  const unsigned U = (unsigned)npan * (unsigned)len;                                          // its units
   const int NST = p.nst;
   const int XST = p.xb * 128 + 16;               // halfs per staged row (row pitch = 32 B mod 128 B)
 
@@ -95,10 +72,9 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
   __half* xs = reinterpret_cast<__half*>(gsum + (((size_t)p.xb * GPB * MP + 1) & ~(size_t)1));  // [m][XST]
   auto tile_of = [&](int w, int which) { return tiles + (size_t)((w * 2 + which) * m) * 32; };
 
-  // ranges of units: CTA [lo, hi), warp [wlo, whi)
-  const unsigned lo = p.panel_cut ? (unsigned)((long)npan * blockIdx.x / G) * (unsigned)nbat : (unsigned)((unsigned long long)U * blockIdx.x / (unsigned)G);
-  const unsigned hi = p.panel_cut ? (unsigned)((long)npan * (blockIdx.x + 1) / G) * (unsigned)nbat
-                                  : (unsigned)((unsigned long long)U * (blockIdx.x + 1) / (unsigned)G);
+  // ranges of units: CTA [lo, hi), warp [wlo, whi); unit u = batch u % len of panel u / len
+  const unsigned lo = p.panel_cut ? (unsigned)npan * cta / G * (unsigned)len : U * cta / G;
+  const unsigned hi = p.panel_cut ? (unsigned)npan * (cta + 1) / G * (unsigned)len : U * (cta + 1) / G;
   const unsigned nu = hi - lo;
   auto warp_lo = [&](int w) { return lo + (unsigned)w * nu / kW8; };
   auto warp_of = [&](unsigned u) { return (int)(((u - lo + 1) * kW8 - 1) / nu); };
@@ -110,11 +86,10 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
   }
   __syncwarp();
   // weights do not depend on the previous kernel: fill the ring before the dependency wait
-  const Cur wc = cur_at(min(wlo, U - 1u), npan, nbat, S);
-  // producer (lane 0): source of the next unit, units left in its segment and in this warp's range
-  Cur pc = wc;
-  const uint8_t* psrc = a.wq + ((size_t)pc.pan * nbat + pc.base + pc.b) * R::BLK;
-  int pseg = pc.len - pc.b, pleft = (int)(whi - wlo);
+  const int wpan = (int)(wlo / (unsigned)len), wb = (int)(wlo - (unsigned)wpan * (unsigned)len);
+  // producer (lane 0): source of the next unit, units left in its panel and in this warp's range
+  const uint8_t* psrc = a.wq + ((size_t)wpan * nbat + base + wb) * R::BLK;
+  int pseg = len - wb, pleft = (int)(whi - wlo);
   uint32_t pdst = ring_u, pbar = bars_u;
   auto issue = [&]() {
     mbar_expect_tx(pbar, (uint32_t)R::BLK);
@@ -124,26 +99,33 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
     if (pbar == bars_u + NST * 8) { pbar = bars_u; pdst = ring_u; }
     psrc += R::BLK;
     --pleft;
-    if (--pseg == 0 && pleft > 0) {
-      pc.b = pc.len - 1;
-      cur_next(pc, npan, nbat, S);
-      psrc = a.wq + ((size_t)pc.pan * nbat + pc.base) * R::BLK;
-      pseg = pc.len;
+    if (--pseg == 0) {           // on to the slice's batches of the next panel
+      psrc += (size_t)(nbat - len) * R::BLK;
+      pseg = len;
     }
   };
   if (lane == 0) {
     for (int i = 0; i < NST && pleft > 0; ++i) issue();
   }
   __syncwarp();
+  // the norm weights of this thread's first two items, too
+  const int nvec = len * 16, total = nvec * m;
+  auto item = [&](int i, int& tok, int& v) { tok = ONE ? 0 : i / nvec; v = i - tok * nvec; };
+  uint4 pre[2], prw[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int i = (int)threadIdx.x + j * kT8;
+    prw[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (a.pro == PRO_NORM && i < total) {
+      int tok, v;
+      item(i, tok, v);
+      prw[j] = *reinterpret_cast<const uint4*>(a.norm_w + base * 128 + v * 8);
+    }
+  }
   pdl_wait();
   pdl_launch_dependents();
 
-  // ---- stage the activations of batches [kA, kB): fp16(x / c) and the per-group sums ----
-  const Cur c0 = cur_at(lo, npan, nbat, S), c1 = cur_at(hi - 1u, npan, nbat, S);
-  const int kA = c0.base, nstage = c1.base + c1.len - kA;
-  const int nvec = nstage * 16, total = nvec * m;
-  auto item = [&](int i, int& tok, int& v) { tok = ONE ? 0 : i / nvec; v = i - tok * nvec; };
-  uint4 pre[2];
+  // ---- stage the activations of the slice: fp16(x / c) and the per-group sums ----
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int i = (int)threadIdx.x + j * kT8;
@@ -151,7 +133,7 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
     if (i < total) {
       int tok, v;
       item(i, tok, v);
-      pre[j] = *reinterpret_cast<const uint4*>(a.x + (size_t)tok * a.ldx + kA * 128 + v * 8);
+      pre[j] = *reinterpret_cast<const uint4*>(a.x + (size_t)tok * a.ldx + base * 128 + v * 8);
     }
   }
   if (a.pro == PRO_NORM) {
@@ -188,7 +170,7 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
 #pragma unroll
         for (int e = 0; e < 8; ++e) f[e] = __bfloat162float(xb[e]);
         if (a.pro == PRO_NORM) {
-          const uint4 wr = *reinterpret_cast<const uint4*>(a.norm_w + kA * 128 + v * 8);
+          const uint4 wr = prw[j];
           const bf16* wb = reinterpret_cast<const bf16*>(&wr);
           const float ir = inv_rms[tok];
 #pragma unroll
@@ -217,7 +199,8 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
       if (in < total) {
         int tk, vn;
         item(in, tk, vn);
-        pre[j] = *reinterpret_cast<const uint4*>(a.x + (size_t)tk * a.ldx + kA * 128 + vn * 8);
+        pre[j] = *reinterpret_cast<const uint4*>(a.x + (size_t)tk * a.ldx + base * 128 + vn * 8);
+        if (a.pro == PRO_NORM) prw[j] = *reinterpret_cast<const uint4*>(a.norm_w + base * 128 + vn * 8);
       }
     }
   }
@@ -280,25 +263,23 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
       }
     }
   };
-  auto cta_of = [&](unsigned u) { return (int)((((unsigned long long)u + 1) * (unsigned)G - 1) / U); };
-  // This CTA's part of segment (slice s, panel pan) is complete in v: the epilogue if that is the whole panel, else the
-  // hand-over through scratch.
-  auto finish = [&](int s, int pan, bool whole, float (&v)[MP]) {
+  // This CTA's part of panel `pan` is complete in v: the epilogue if that is the whole panel, else the hand-over through
+  // scratch.
+  auto finish = [&](int pan, bool whole, float (&v)[MP]) {
     if (whole && S == 1) { epilogue(pan, v); return; }
-    // lane l: CTAs that share segment (l, pan)
+    // lane l: CTAs of slice l that share the panel.  The CTA of unit u is the last whose range begins at or before it.
     int first = 0, cnt = 0;
     if (lane < S) {
-      const int sb = slice_base(lane, nbat, S), len = slice_base(lane + 1, nbat, S) - sb;
-      const unsigned u0 = (unsigned)npan * (unsigned)sb + (unsigned)pan * (unsigned)len;
-      first = cta_of(u0);
-      cnt = cta_of(u0 + (unsigned)len - 1u) - first + 1;
+      const unsigned ll = (unsigned)(slice_base(lane + 1, nbat, S) - slice_base(lane, nbat, S)), Ul = (unsigned)npan * ll;
+      first = (int)((((unsigned)pan * ll + 1u) * G - 1u) / Ul);
+      cnt = (int)((((unsigned)pan + 1u) * ll * G - 1u) / Ul) - first + 1;
     }
-    const int my_first = __shfl_sync(0xffffffffu, first, s);
+    const int my_first = __shfl_sync(0xffffffffu, first, slice);
     int nparts = cnt;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) nparts += __shfl_xor_sync(0xffffffffu, nparts, o);
     const size_t tsz = (size_t)m * 32;
-    float* mine = a.scratch + (((size_t)s * npan + pan) * p.fmax + ((int)blockIdx.x - my_first)) * tsz + lane;
+    float* mine = a.scratch + (((size_t)slice * npan + pan) * p.fmax + ((int)cta - my_first)) * tsz + lane;
 #pragma unroll
     for (int tok = 0; tok < MP; ++tok)
       if (tok < m) mine[tok * 32] = v[tok];
@@ -337,21 +318,18 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
   };
 
   // ---- main loop over this warp's units ----
-  Cur cc = wc;
   const uint8_t* cptr = ring;
   uint32_t cbar = bars_u, cph = 0;
   bool failed = false;
   const bool tok_ok = g < m;
-  for (unsigned u = wlo; u < whi && !failed;) {
-    // one fragment: the units of segment (cc.s, cc.pan) inside [u, whi)
-    const int s = cc.s, pan = cc.pan;
-    const unsigned seg0 = u - (unsigned)cc.b, seg1 = seg0 + (unsigned)cc.len;     // units of the whole segment
+  int pan = wpan, b0 = wb;
+  for (unsigned u = wlo; u < whi && !failed; ++pan, b0 = 0) {
+    // one fragment: the units of this panel inside [u, whi)
+    const unsigned seg0 = (unsigned)pan * (unsigned)len, seg1 = seg0 + (unsigned)len;
     const int cnt = (int)(min(seg1, whi) - u);
-    const __half* xrow = xs + (size_t)(ONE ? 0 : (tok_ok ? g : 0)) * XST + (cc.base - kA + cc.b) * 128 + t * 4;
-    const float2* gs = gsum + (size_t)((cc.base - kA + cc.b) * GPB) * MP + (ONE ? 0 : 2 * t);
+    const __half* xrow = xs + (size_t)(ONE ? 0 : (tok_ok ? g : 0)) * XST + b0 * 128 + t * 4;
+    const float2* gs = gsum + (size_t)(b0 * GPB) * MP + (ONE ? 0 : 2 * t);
     u += (unsigned)cnt;
-    cc.b = cc.len - 1;                            // the cursor moves on to the next segment
-    cur_next(cc, npan, nbat, S);
     float y[2][4];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
@@ -431,7 +409,7 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
 #pragma unroll
       for (int tok = 0; tok < MP; ++tok) v[tok] = tok < m ? tile[tok * 32 + lane] : 0.f;
       __syncwarp();
-      finish(s, pan, seg0 >= lo && seg1 <= hi, v);
+      finish(pan, seg0 >= lo && seg1 <= hi, v);
     }
   }
   const bool any_failed = __syncthreads_or(failed ? 1 : 0) != 0;
@@ -442,52 +420,36 @@ __global__ void __launch_bounds__(kT8, 2) wq_gemv8_kernel(const WqGemvArgs a, co
     return;
   }
   // ---- segments that several warps share: segment j of the CTA is added up by warp j % 16 ----
-  Cur sc = c0;
-  unsigned seg0 = lo - (unsigned)c0.b;
-  for (int j = 0; seg0 < hi; ++j) {
-    const unsigned seg1 = seg0 + (unsigned)sc.len;
-    if ((j & (kW8 - 1)) == warp) {
-      const unsigned a0 = max(seg0, lo), a1 = min(seg1, hi);
-      const int wa = warp_of(a0), wb = warp_of(a1 - 1u);
-      if (wa != wb) {
-        float v[MP];
+  for (int pn = (int)(lo / (unsigned)len) + warp; (unsigned)pn * (unsigned)len < hi; pn += kW8) {
+    const unsigned seg0 = (unsigned)pn * (unsigned)len, seg1 = seg0 + (unsigned)len;
+    const unsigned a0 = max(seg0, lo), a1 = min(seg1, hi);
+    const int wa = warp_of(a0), wz = warp_of(a1 - 1u);
+    if (wa == wz) continue;
+    float v[MP];
 #pragma unroll
-        for (int tok = 0; tok < MP; ++tok) v[tok] = 0.f;
-        for (int w = wa; w <= wb; ++w) {
-          const float* tile = tile_of(w, a0 <= warp_lo(w) ? 0 : 1);
-          if (warp_lo(w) == warp_lo(w + 1)) continue;                             // a warp without units
+    for (int tok = 0; tok < MP; ++tok) v[tok] = 0.f;
+    for (int w = wa; w <= wz; ++w) {
+      if (warp_lo(w) == warp_lo(w + 1)) continue;                                 // a warp without units
+      const float* tile = tile_of(w, a0 <= warp_lo(w) ? 0 : 1);
 #pragma unroll
-          for (int tok = 0; tok < MP; ++tok)
-            if (tok < m) v[tok] += tile[tok * 32 + lane];
-        }
-        finish(sc.s, sc.pan, seg0 >= lo && seg1 <= hi, v);
-      }
+      for (int tok = 0; tok < MP; ++tok)
+        if (tok < m) v[tok] += tile[tok * 32 + lane];
     }
-    seg0 = seg1;
-    sc.b = sc.len - 1;
-    if (seg0 < hi) cur_next(sc, npan, nbat, S);
+    finish(pn, seg0 >= lo && seg1 <= hi, v);
   }
 }
 
-static int g8_ctas(int n, int k, int& slices, int& panel_cut) {
-  const long npan = n / 32, nbat = k / 128, U = npan * nbat;
-  slices = (int)(nbat <= 40 ? 1 : (nbat + 19) / 20);
-  long G = U / kW8;                               // at least one unit per warp
-  if (G < 1) G = 1;
-  const long seg = npan * (nbat / slices);        // a CTA touches two slices at most
-  if (slices > 1 && (U + seg - 1) / seg > G) G = (U + seg - 1) / seg;
-  if (G > 148) G = 148;
-  panel_cut = slices == 1 && npan >= 8 * G;
-  return (int)G;
-}
 static Gemv8Plan g8_plan(int n, int k) {
-  Gemv8Plan p;
-  p.ctas = g8_ctas(n, k, p.slices, p.panel_cut);
-  const long nbat = k / 128, U = (long)(n / 32) * nbat;
-  const long len = (nbat + p.slices - 1) / p.slices, per = U / p.ctas;
-  p.fmax = p.panel_cut ? 1 : (int)((len + per - 1) / per + 1);
-  p.xb = (int)(p.slices == 1 ? nbat : 2 * len);
-  p.nst = 0;
+  Gemv8Plan p = {};
+  const long npan = n / 32, nbat = k / 128;
+  p.slices = (int)((nbat + 39) / 40);
+  long G = npan * nbat / kW8;                     // at least one unit per warp
+  G = G > 148 ? 148 : G;
+  p.per_slice = (int)(G / p.slices < 1 ? 1 : G / p.slices);
+  p.panel_cut = p.slices == 1 && npan >= 8L * p.per_slice;
+  p.xb = (int)((nbat + p.slices - 1) / p.slices);
+  const long per = npan * (nbat / p.slices) / p.per_slice;      // units of a CTA, at least
+  p.fmax = p.panel_cut ? 1 : (int)((p.xb + per - 1) / (per < 1 ? 1 : per) + 1);
   return p;
 }
 
@@ -495,20 +457,17 @@ template <int BITS, int GROUP, bool ONE>
 static int g8_launch(const WqGemvArgs& a, Gemv8Plan p, cudaStream_t st) {
   using R = Ring<BITS, GROUP, 2>;
   constexpr int GPB = 128 / GROUP, MP = ONE ? 1 : 8;
-  // rings of about 5 KB a warp let two kernels share an SM; when the activations are too large for that anyway, 8 KB
+  // Rings of 6.5 KB a warp, 104 KB an SM: 4.4 KB and 8.7 KB measured 10 and 1 % slower.
   const size_t rest = 32 + (size_t)kW8 * 2 * a.m * 32 * 4 + (((size_t)p.xb * GPB * MP + 1) & ~(size_t)1) * 8 + (size_t)a.m * (p.xb * 128 + 16) * 2;
   auto total = [&](int nst) { return (size_t)kW8 * nst * (R::BLK + 8) + rest; };
-  p.nst = 5120 / R::BLK < 2 ? 2 : 5120 / R::BLK;
-  if (total(p.nst) > 112 * 1024) {
-    const int deep = 8704 / R::BLK;
-    p.nst = total(deep) <= 220 * 1024 ? deep : p.nst;
-  }
+  p.nst = 6656 / R::BLK;
+  while (total(p.nst) > 220 * 1024 && p.nst > 2) --p.nst;
   const size_t smem = total(p.nst);
   if (smem > 220 * 1024) return B2_ERR_ARG;
   auto kern = wq_gemv8_kernel<BITS, GROUP, ONE>;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024) != cudaSuccess) return B2_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)p.ctas, 1, 1);
+  cfg.gridDim = dim3((unsigned)(p.slices * p.per_slice), 1, 1);
   cfg.blockDim = dim3(kT8, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
@@ -540,7 +499,7 @@ B2_API int b2_wq_gemv8(const WqGemvArgs* args, cudaStream_t stream) {
   if (a.ks < 1 || a.ks > kMaxKs || a.k / 128 % a.ks || (a.rb != 2 && a.rb != 4)) return B2_ERR_ARG;   // a linear that the other kernel takes
   if (!a.scratch || !a.counters || a.epi == EPI_TP_RESID) return B2_ERR_ARG;
   if ((a.ldx % 8) || (reinterpret_cast<uintptr_t>(a.x) & 15)) return B2_ERR_ARG;
-  if ((double)(a.n / 32) * (double)(a.k / 128) * kW8 >= 4.0e9) return B2_ERR_ARG;   // 32-bit schedule arithmetic
+  if ((double)(a.n / 32) * (double)(a.k / 128) * 148.0 >= 4.0e9) return B2_ERR_ARG;   // 32-bit schedule arithmetic
   const Gemv8Plan p = g8_plan(a.n, a.k);
   if (p.slices > 32) return B2_ERR_ARG;
   for (int t0 = 0; t0 < a.m; t0 += 8) {
