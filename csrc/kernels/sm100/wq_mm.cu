@@ -246,20 +246,24 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
 
   if (warp == 0) {
     // ---------------- packed weights ----------------
-    if (lane == 0) {
-      int tile = tile0, kb = kb0;
-      RingPos r;
-      for (int i = 0; i < nu; ++i, r.next(RS)) {
-        if (i >= RS && !mbar_wait_bounded(smem_u32(&raw_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
-        const uint32_t bar = smem_u32(&raw_full[r.s]);
-        mbar_expect_tx(bar, (uint32_t)RAW);
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const int pan = min(tile * 4 + p, npan - 1);       // a ragged last tile repeats the last panel; its rows are never stored
-          bulk_g2s(raw_ring + (uint32_t)(r.s * RAW + p * R::BLK), a.wq + ((size_t)pan * nbat + kb) * R::BLK, (uint32_t)R::BLK, bar);
-        }
-        if (++kb == nbat) { kb = 0; ++tile; }
+    // lane p < 4 copies panel p of every unit
+    int left = nbat - kb0, tile = tile0;
+    const uint8_t* src = a.wq + ((size_t)min(tile * 4 + (lane & 3), npan - 1) * nbat + kb0) * R::BLK;
+    uint32_t full = smem_u32(&raw_full[0]), empty = smem_u32(&raw_empty[0]), dst = raw_ring + (uint32_t)((lane & 3) * R::BLK);
+    uint32_t ph = 1;
+    for (int i = 0, s = 0; i < nu; ++i) {
+      if (i >= RS && !mbar_wait_warp(empty, ph)) { atomicExch(&s_failed, 1); break; }
+      if (lane == 0) mbar_expect_tx(full, (uint32_t)RAW);
+      __syncwarp();
+      if (lane < 4) bulk_g2s(dst, src, (uint32_t)R::BLK, full);
+      src += R::BLK;
+      if (--left == 0) {             // a ragged last tile repeats the last panel; its rows are never stored
+        left = nbat;
+        ++tile;
+        src = a.wq + (size_t)min(tile * 4 + (lane & 3), npan - 1) * nbat * R::BLK;
       }
+      full += 8; empty += 8; dst += RAW;
+      if (++s == RS) { s = 0; ph ^= 1u; full -= RS * 8; empty -= RS * 8; dst -= RS * RAW; }
     }
   } else if (warp == 2) {
     // ---------------- activation tiles by TMA (written by the previous kernel) ----------------
@@ -281,23 +285,39 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
       const uint32_t idesc = idesc_f16(BM, a.n_pad);
-      int kb = kb0, frag = 0;
-      RingPos r, d;
-      const uint64_t dx_base = desc_sw128(x_ring);          // stages are 2 x_sub bytes apart; the field counts 16 bytes
+      // a lone thread's loop: every instruction costs several cycles, so addresses advance by additions
+      const uint64_t dx_base = desc_sw128(x_ring);          // the address field counts 16 bytes
       const uint32_t dx_step = (2 * x_sub) >> 4, dx_half = x_sub >> 4;
-      for (int i = 0; i < nu; ++i, r.next(NB)) {
-        const bool first = i == 0 || kb == 0, last = i == nu - 1 || kb == nbat - 1;
-        if (first && frag >= nd && !mbar_wait_bounded(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
-        if (!mbar_wait_bounded(smem_u32(&op_full[r.s]), r.ph)) { atomicExch(&s_failed, 1); break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t dx = dx_base + (uint32_t)r.s * dx_step;
-        const uint32_t ta = tmem_base + (uint32_t)(r.s * 64), td = tmem_d0 + (uint32_t)(d.s * a.n_pad);
+      const uint32_t full0 = smem_u32(&op_full[0]), empty0 = smem_u32(&op_empty[0]), wrap = (uint32_t)NB * 8;
+      uint32_t off = 0, ph = 0, ta = tmem_base;
+      uint64_t dx = dx_base;
+      RingPos d;
+      bool ok = true;
+      int kb = kb0;
+      for (int left = nu, frag = 0; left > 0 && ok; ++frag, d.next(nd)) {
+        int cnt = min(nbat - kb, left);
+        left -= cnt;
+        kb = 0;
+        if (frag >= nd && !mbar_wait_bounded(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { ok = false; break; }
+        const uint32_t td = tmem_d0 + (uint32_t)(d.s * a.n_pad);
+        uint32_t acc = 0;
+        for (; cnt > 0; --cnt) {
+          if (!mbar_wait_bounded(full0 + off, ph)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          umma_f16(td, ta, dx, idesc, acc);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) umma_f16(td, ta + q * 8, dx + (q < 4 ? 0u : dx_half) + 2 * (q & 3), idesc, (!first || q) ? 1u : 0u);
-        umma_commit_m(smem_u32(&op_empty[r.s]));
-        if (last) { umma_commit_m(smem_u32(&d_full[d.s])); ++frag; d.next(nd); }
-        if (++kb == nbat) kb = 0;
+          for (int q = 1; q < 4; ++q) umma_f16(td, ta + q * 8, dx + 2 * q, idesc, 1u);
+          const uint64_t dh = dx + dx_half;
+#pragma unroll
+          for (int q = 0; q < 4; ++q) umma_f16(td, ta + 32 + q * 8, dh + 2 * q, idesc, 1u);
+          umma_commit_m(empty0 + off);
+          acc = 1u;
+          off += 8; ta += 64; dx += dx_step;
+          if (off == wrap) { off = 0; ta = tmem_base; dx = dx_base; ph ^= 1u; }
+        }
+        umma_commit_m(smem_u32(&d_full[d.s]));
       }
+      if (!ok) atomicExch(&s_failed, 1);
     }
   } else if (warp >= kDqWarp0) {
     // ---------------- dequantisers: panel warp % 4 of every third unit ----------------
