@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
   __shared__ int s_failed;
   __shared__ unsigned s_prev;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int RS = a.raw_stages;
   const uint32_t x_sub = (uint32_t)a.n_pad * BKS * 2;
   const uint32_t x_ring = (smem_u32(smem_m) + 1023u) & ~1023u;                     // [NB][2 halves of k][n_pad rows][128 B]
@@ -283,42 +283,44 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      const uint32_t idesc = idesc_f16(BM, a.n_pad);
-      // a lone thread's loop: every instruction costs several cycles, so addresses advance by additions
-      const uint64_t dx_base = desc_sw128(x_ring);          // the address field counts 16 bytes
-      const uint32_t dx_step = (2 * x_sub) >> 4, dx_half = x_sub >> 4;
-      const uint32_t full0 = smem_u32(&op_full[0]), empty0 = smem_u32(&op_empty[0]), wrap = (uint32_t)NB * 8;
-      uint32_t off = 0, ph = 0, ta = tmem_base;
-      uint64_t dx = dx_base;
-      RingPos d;
-      bool ok = true;
-      int kb = kb0;
-      for (int left = nu, frag = 0; left > 0 && ok; ++frag, d.next(nd)) {
-        int cnt = min(nbat - kb, left);
-        left -= cnt;
-        kb = 0;
-        if (frag >= nd && !mbar_wait_bounded(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { ok = false; break; }
-        const uint32_t td = tmem_d0 + (uint32_t)(d.s * a.n_pad);
-        uint32_t acc = 0;
-        for (; cnt > 0; --cnt) {
-          if (!mbar_wait_bounded(full0 + off, ph)) { ok = false; break; }
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // The whole warp runs the loop and its first lane issues: addresses then stay in uniform registers, which tcgen05.mma
+    // takes its operands from (under `if (lane == 0)` around the loop an MMA took 70 cycles to issue, 1050 a unit).
+    const uint32_t idesc = idesc_f16(BM, a.n_pad);
+    const uint64_t dx_base = desc_sw128(x_ring);            // the address field counts 16 bytes
+    const uint32_t dx_step = (2 * x_sub) >> 4, dx_half = x_sub >> 4;
+    const uint32_t full0 = smem_u32(&op_full[0]), empty0 = smem_u32(&op_empty[0]), wrap = (uint32_t)NB * 8;
+    uint32_t off = 0, ph = 0, ta = tmem_base;
+    uint64_t dx = dx_base;
+    RingPos d;
+    bool ok = true;
+    int kb = kb0;
+    for (int left = nu, frag = 0; left > 0 && ok; ++frag, d.next(nd)) {
+      int cnt = min(nbat - kb, left);
+      left -= cnt;
+      kb = 0;
+      if (frag >= nd && !mbar_wait_warp(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { ok = false; break; }
+      const uint32_t td = tmem_d0 + (uint32_t)(d.s * a.n_pad);
+      uint32_t acc = 0;
+      for (; cnt > 0; --cnt) {
+        if (!mbar_wait_warp(full0 + off, ph)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t dh = dx + dx_half;
+        if (lane == 0) {
           umma_f16(td, ta, dx, idesc, acc);
 #pragma unroll
           for (int q = 1; q < 4; ++q) umma_f16(td, ta + q * 8, dx + 2 * q, idesc, 1u);
-          const uint64_t dh = dx + dx_half;
 #pragma unroll
           for (int q = 0; q < 4; ++q) umma_f16(td, ta + 32 + q * 8, dh + 2 * q, idesc, 1u);
           umma_commit_m(empty0 + off);
-          acc = 1u;
-          off += 8; ta += 64; dx += dx_step;
-          if (off == wrap) { off = 0; ta = tmem_base; dx = dx_base; ph ^= 1u; }
+          if (cnt == 1) umma_commit_m(smem_u32(&d_full[d.s]));
         }
-        umma_commit_m(smem_u32(&d_full[d.s]));
+        __syncwarp();
+        acc = 1u;
+        off += 8; ta += 64; dx += dx_step;
+        if (off == wrap) { off = 0; ta = tmem_base; dx = dx_base; ph ^= 1u; }
       }
-      if (!ok) atomicExch(&s_failed, 1);
     }
+    if (!ok) s_failed = 1;
   } else if (warp >= kDqWarp0) {
     // ---------------- dequantisers: panel warp % 4 of every third unit ----------------
     const int p = warp & 3;
