@@ -141,7 +141,7 @@ class WqMmArgs(C.Structure):
     _fields_ = [
         ("wq", C.c_void_p), ("n", C.c_int), ("k", C.c_int), ("m", C.c_int),
         ("bits", C.c_int), ("group", C.c_int),
-        ("ctas", C.c_int), ("n_pad", C.c_int), ("raw_stages", C.c_int), ("bufs", C.c_int),
+        ("ctas", C.c_int), ("n_pad", C.c_int), ("per", C.c_int), ("raw_stages", C.c_int), ("bufs", C.c_int),
         ("epi", C.c_int),
         ("y", C.c_void_p), ("ldy", C.c_long),
         ("resid", C.c_void_p), ("ldr", C.c_long),

@@ -8,7 +8,7 @@
 // the contiguous range [c U / G, (c + 1) U / G) of it, so every SM has the same share for every shape.  Per CTA:
 //   warp 0       bulk copies of the packed weights (four 32-row panels a unit) into a ring of shared-memory stages; they do
 //                not depend on the previous kernel and start before the dependency wait
-//   warp 1       one elected thread issues tcgen05.mma (kind f16, A in TMEM, B in shared memory, fp32 accumulator in TMEM)
+//   warp 1       its first lane issues tcgen05.mma (kind f16, A in TMEM, B in shared memory, fp32 accumulator in TMEM)
 //   warp 2       TMA: fp16 activation tiles [tokens][64 k] (128-byte swizzle)
 //   warps 4-11   epilogue (store, residual + next-norm statistics, SwiGLU, fp32, argmax partials as in the GEMV): two
 //                warps per 32 TMEM lanes, half of the tokens each; accumulators are double-buffered up to 128 tokens
@@ -19,12 +19,13 @@
 // Replaces dequant_kt_kernel + cuBLAS and w4_gemm_kernel / w4h_bt_kernel of the reference
 // (kernels/m1/m1_model.cu:1875-1895, kernels/src/w4_gemv.cu, w4h.cu) for every m above the GEMV's range.
 //
-// What bounds it: up to about 64 tokens the MMA issuer's loop (some 1200 cycles a unit, most of it moving the operands of
-// eight tcgen05.mma to uniform registers; the packed weights of a 4-bit unit need 380 at the copy rate), beyond that the
-// activation tiles, which every CTA reads from L2 (256 tokens: 64 KB a unit).  The earlier kernel wrote fp16 tiles to
-// shared memory from a register ring and cut k into equal slices (80 tiles x 2 slices = two waves of 148).  4 bits,
-// graph replays over weights larger than L2, before -> now: 24 tokens qkv 55 -> 24 us, o 49 -> 22, gate_up 105 -> 77,
-// down 94 -> 48; 256 tokens qkv 215 -> 49, o 211 -> 51, gate_up 222 -> 127 (1058 TFLOP/s), down 268 -> 84.
+// What bounds it: up to about 64 tokens the pace of the issuing warps (some 650 cycles a unit; two units are one pipeline
+// step there, one barrier round for sixteen MMAs), beyond that the MMAs (256 tokens: 1024 cycles a unit at the nominal
+// rate) and, above 128 tokens, the epilogue of a tile, since only one such accumulator fits TMEM.  The earlier kernel wrote
+// fp16 tiles to shared memory from a register ring and cut k into equal slices (80 tiles x 2 slices = two waves of 148).
+// 4 bits, graph replays over weights larger than L2, before -> now: 16 tokens qkv 55 -> 21 us, o 49 -> 19, gate_up 105 ->
+// 54, down 94 -> 34, lm_head 303 -> 137; 256 tokens qkv 215 -> 46, o 211 -> 49, gate_up 222 -> 120 (1120 TFLOP/s), down
+// 268 -> 79, lm_head 655 -> 320 (1250 TFLOP/s).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -37,6 +38,7 @@ struct WqMmArgs {
   int bits, group;
   int ctas;                   // b2_wq_mm_ctas(n, k)
   int n_pad;                  // token rows of the fp16 activation buffer: b2_wq_mm_npad(m)
+  int per;                    // units of a pipeline step: 2 up to 64 tokens, else 1
   int raw_stages, bufs;       // shared-memory stages of packed weights; operand buffers (weights in TMEM, activations in shared memory)
   int epi;
   bf16* y; long ldy;
@@ -54,7 +56,7 @@ enum { EPI_STORE = 0, EPI_RESID = 1, EPI_SWIGLU = 2, EPI_F32 = 3, EPI_ARGMAX = 4
 constexpr int BM = 128, BKS = 64;                // BKS: width of one 128-byte swizzle atom in fp16 elements
 constexpr int kMmThreads = 768;                  // 24 warps: weights, MMA, activations, spare, 8 epilogue, 12 dequantisers
 constexpr int kEpiWarp0 = 4, kEpiWarps = 8, kDqWarp0 = 12, kDqSets = 3;
-constexpr int kMaxRaw = 16, kMaxBuf = 6;
+constexpr int kMaxRaw = 16, kMaxBuf = 4;
 constexpr int kTmemColsM = 512;
 
 __device__ __forceinline__ void mbar_arrive_m(uint32_t bar) {
@@ -215,9 +217,10 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
   const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int RS = a.raw_stages;
   const uint32_t x_sub = (uint32_t)a.n_pad * BKS * 2;
-  const uint32_t x_ring = (smem_u32(smem_m) + 1023u) & ~1023u;                     // [NB][2 halves of k][n_pad rows][128 B]
-  const int NB = a.bufs;
-  const uint32_t raw_ring = x_ring + (uint32_t)NB * 2 * x_sub;
+  const int P = a.per, NB = a.bufs;
+  const uint32_t x_step = (uint32_t)P * 2 * x_sub, raw_step = (uint32_t)(P * RAW);
+  const uint32_t x_ring = (smem_u32(smem_m) + 1023u) & ~1023u;                     // [NB][P][2 halves of k][n_pad rows][128 B]
+  const uint32_t raw_ring = x_ring + (uint32_t)NB * x_step;                        // [RS][4 panels][P][block]
   uint8_t* raw_ptr = smem_m + (raw_ring - smem_u32(smem_m));
   const int nbat = a.k / 128, npan = a.n / 32;
   const int tiles = (a.n + BM - 1) / BM;
@@ -242,28 +245,31 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = tmem_slot;
-  const uint32_t tmem_d0 = tmem_base + (uint32_t)NB * 64;
+  const uint32_t tmem_d0 = tmem_base + (uint32_t)(NB * P) * 64;
 
   if (warp == 0) {
     // ---------------- packed weights ----------------
-    // lane p < 4 copies panel p of every unit
+    // lane p < 4 copies panel p of every step
     int left = nbat - kb0, tile = tile0;
     const uint8_t* src = a.wq + ((size_t)min(tile * 4 + (lane & 3), npan - 1) * nbat + kb0) * R::BLK;
-    uint32_t full = smem_u32(&raw_full[0]), empty = smem_u32(&raw_empty[0]), dst = raw_ring + (uint32_t)((lane & 3) * R::BLK);
+    uint32_t full = smem_u32(&raw_full[0]), empty = smem_u32(&raw_empty[0]), dst = raw_ring + (uint32_t)((lane & 3) * P * R::BLK);
     uint32_t ph = 1;
-    for (int i = 0, s = 0; i < nu; ++i) {
-      if (i >= RS && !mbar_wait_warp(empty, ph)) { atomicExch(&s_failed, 1); break; }
-      if (lane == 0) mbar_expect_tx(full, (uint32_t)RAW);
+    for (int i = 0, st = 0, s = 0; i < nu; ++st) {
+      const int cnt = min(P, min(left, nu - i));
+      if (st >= RS && !mbar_wait_warp(empty, ph)) { atomicExch(&s_failed, 1); break; }
+      if (lane == 0) mbar_expect_tx(full, (uint32_t)(cnt * RAW));
       __syncwarp();
-      if (lane < 4) bulk_g2s(dst, src, (uint32_t)R::BLK, full);
-      src += R::BLK;
-      if (--left == 0) {             // a ragged last tile repeats the last panel; its rows are never stored
+      if (lane < 4) bulk_g2s(dst, src, (uint32_t)(cnt * R::BLK), full);
+      i += cnt;
+      src += cnt * R::BLK;
+      left -= cnt;
+      if (left == 0) {               // a ragged last tile repeats the last panel; its rows are never stored
         left = nbat;
         ++tile;
         src = a.wq + (size_t)min(tile * 4 + (lane & 3), npan - 1) * nbat * R::BLK;
       }
-      full += 8; empty += 8; dst += RAW;
-      if (++s == RS) { s = 0; ph ^= 1u; full -= RS * 8; empty -= RS * 8; dst -= RS * RAW; }
+      full += 8; empty += 8; dst += raw_step;
+      if (++s == RS) { s = 0; ph ^= 1u; full -= RS * 8; empty -= RS * 8; dst -= RS * raw_step; }
     }
   } else if (warp == 2) {
     // ---------------- activation tiles by TMA (written by the previous kernel) ----------------
@@ -272,13 +278,15 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       pdl_launch_dependents();
       int kb = kb0;
       RingPos r;
-      for (int i = 0; i < nu; ++i, r.next(NB)) {
-        if (i >= NB && !mbar_wait_bounded(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
+      for (int i = 0, st = 0; i < nu; ++st, r.next(NB)) {
+        const int cnt = min(P, min(nbat - kb, nu - i));
+        if (st >= NB && !mbar_wait_bounded(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
         const uint32_t bar = smem_u32(&op_full[r.s]);
-        mbar_expect_tx(bar, 2 * x_sub);
-        tma_load_2d_m(x_ring + 2 * r.s * x_sub, &map_x, kb * 128, 0, bar);
-        tma_load_2d_m(x_ring + (2 * r.s + 1) * x_sub, &map_x, kb * 128 + BKS, 0, bar);
-        if (++kb == nbat) kb = 0;
+        mbar_expect_tx(bar, (uint32_t)cnt * 2 * x_sub);
+        for (int h = 0; h < 2 * cnt; ++h) tma_load_2d_m(x_ring + r.s * x_step + h * x_sub, &map_x, kb * 128 + h * BKS, 0, bar);
+        i += cnt;
+        kb += cnt;
+        if (kb == nbat) kb = 0;
       }
     }
   } else if (warp == 1) {
@@ -287,7 +295,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
     // takes its operands from (under `if (lane == 0)` around the loop an MMA took 70 cycles to issue, 1050 a unit).
     const uint32_t idesc = idesc_f16(BM, a.n_pad);
     const uint64_t dx_base = desc_sw128(x_ring);            // the address field counts 16 bytes
-    const uint32_t dx_step = (2 * x_sub) >> 4, dx_half = x_sub >> 4;
+    const uint32_t dx_half = x_sub >> 4, dx_step = x_step >> 4, ta_step = (uint32_t)P * 64;
     const uint32_t full0 = smem_u32(&op_full[0]), empty0 = smem_u32(&op_empty[0]), wrap = (uint32_t)NB * 8;
     uint32_t off = 0, ph = 0, ta = tmem_base;
     uint64_t dx = dx_base;
@@ -301,22 +309,30 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       if (frag >= nd && !mbar_wait_warp(smem_u32(&d_empty[d.s]), d.ph ^ 1u)) { ok = false; break; }
       const uint32_t td = tmem_d0 + (uint32_t)(d.s * a.n_pad);
       uint32_t acc = 0;
-      for (; cnt > 0; --cnt) {
+      while (cnt > 0) {
+        const int c = min(P, cnt);
+        cnt -= c;
         if (!mbar_wait_warp(full0 + off, ph)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint64_t dh = dx + dx_half;
+        const uint64_t dh = dx + dx_half, dy = dh + dx_half, dz = dy + dx_half;
         if (lane == 0) {
           umma_f16(td, ta, dx, idesc, acc);
 #pragma unroll
           for (int q = 1; q < 4; ++q) umma_f16(td, ta + q * 8, dx + 2 * q, idesc, 1u);
 #pragma unroll
           for (int q = 0; q < 4; ++q) umma_f16(td, ta + 32 + q * 8, dh + 2 * q, idesc, 1u);
+          if (c == 2) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) umma_f16(td, ta + 64 + q * 8, dy + 2 * q, idesc, 1u);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) umma_f16(td, ta + 96 + q * 8, dz + 2 * q, idesc, 1u);
+          }
           umma_commit_m(empty0 + off);
-          if (cnt == 1) umma_commit_m(smem_u32(&d_full[d.s]));
+          if (cnt == 0) umma_commit_m(smem_u32(&d_full[d.s]));
         }
         __syncwarp();
         acc = 1u;
-        off += 8; ta += 64; dx += dx_step;
+        off += 8; ta += ta_step; dx += dx_step;
         if (off == wrap) { off = 0; ta = tmem_base; dx = dx_base; ph ^= 1u; }
       }
     }
@@ -328,29 +344,45 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
     RingPos rw, rb;
     rw.next(RS, set);
     rb.next(NB, set);
-    for (int i = set; i < nu; i += kDqSets, rw.next(RS, kDqSets), rb.next(NB, kDqSets)) {
-      const int b = rb.s;
+    int kb = kb0, st = 0, turn = 0;
+    for (int i = 0; i < nu; ++st) {
+      const int cnt = min(P, min(nbat - kb, nu - i));
+      i += cnt;
+      kb += cnt;
+      if (kb == nbat) kb = 0;
+      const bool mine = turn == set;                        // the sets take the steps in turn
+      if (++turn == kDqSets) turn = 0;
+      if (!mine) continue;
       if (!mbar_wait_warp(smem_u32(&raw_full[rw.s]), rw.ph)) { atomicExch(&s_failed, 1); break; }
-      const uint8_t* blk = raw_ptr + rw.s * RAW + p * R::BLK;
-      WFrag<BITS, GROUP> f[2];
+      bool ok = true;
+      const uint8_t* blk = raw_ptr + rw.s * raw_step + p * P * R::BLK;
+      for (int c = 0; c < cnt; ++c, blk += R::BLK) {
+        WFrag<BITS, GROUP> f[2];
 #pragma unroll
-      for (int r = 0; r < 2; ++r) load_frag_smem<BITS, GROUP>(f[r], blk + r * R::W_BATCH, blk + 2 * R::W_BATCH + r * GPB * 64, lane);
-      __syncwarp();
-      if (lane == 0) mbar_arrive_m(smem_u32(&raw_empty[rw.s]));
-      if (i >= NB) {
-        if (!mbar_wait_warp(smem_u32(&op_empty[b]), rb.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      }
+        for (int r = 0; r < 2; ++r) load_frag_smem<BITS, GROUP>(f[r], blk + r * R::W_BATCH, blk + 2 * R::W_BATCH + r * GPB * 64, lane);
+        if (c == cnt - 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive_m(smem_u32(&raw_empty[rw.s]));
+        }
+        if (c == 0 && st >= NB) {                           // the packed words are in registers before this wait
+          ok = mbar_wait_warp(smem_u32(&op_empty[rb.s]), rb.ph ^ 1u);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          if (!ok) break;
+        }
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        uint32_t w[32];
-        dequant_frag<BITS, GROUP>(f[r], w);
-        tmem_st_frag(tmem_base + ((uint32_t)(p * 32 + r * 16) << 16) + (uint32_t)(b * 64), w);
+        for (int r = 0; r < 2; ++r) {
+          uint32_t w[32];
+          dequant_frag<BITS, GROUP>(f[r], w);
+          tmem_st_frag(tmem_base + ((uint32_t)(p * 32 + r * 16) << 16) + (uint32_t)((rb.s * P + c) * 64), w);
+        }
       }
+      if (!ok) { atomicExch(&s_failed, 1); break; }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) mbar_arrive_m(smem_u32(&op_full[b]));
+      if (lane == 0) mbar_arrive_m(smem_u32(&op_full[rb.s]));
+      rw.next(RS, kDqSets);
+      rb.next(NB, kDqSets);
     }
   } else if (warp >= kEpiWarp0) {
     // ---------------- epilogue: TMEM lanes 32 (warp % 4), token half (warp - 4) / 4 ----------------
@@ -545,9 +577,12 @@ B2_API int b2_wq_mm(const WqMmArgs* args, const bf16* x, long ldx, const float* 
   // packed weights (what is left above 160 tokens, whose activation tiles are large)
   const int raw = 8 * (a.bits == 3 ? 768 : (a.bits == 4 ? 1024 : 512)) + 8 * (128 / a.group) * 64;
   const int x_sub = a.n_pad * BKS * 2;
-  a.bufs = a.n_pad <= 64 ? 6 : (a.n_pad <= 160 ? 4 : 3);
-  const int left = 220 * 1024 - a.bufs * 2 * x_sub;
-  a.raw_stages = (left < 64 * 1024 ? left : 64 * 1024) / raw;
+  // A step of two units halves the issuing warps' cost per unit; its three buffers take 384 TMEM columns, which leaves two
+  // accumulators of 64 tokens.
+  a.per = a.n_pad <= 64 ? 2 : 1;
+  a.bufs = a.n_pad <= 64 ? 3 : (a.n_pad <= 160 ? 4 : 3);
+  const int left = 220 * 1024 - a.bufs * a.per * 2 * x_sub;
+  a.raw_stages = (left < 80 * 1024 ? left : 80 * 1024) / (a.per * raw);
   if (a.raw_stages > kMaxRaw) a.raw_stages = kMaxRaw;
   // A multiple of the dequantiser sets: a stage is then always read by the same set, which has seen its previous phase
   // complete before it waits for the next (a parity wait must not come a phase early).
@@ -572,7 +607,7 @@ B2_API int b2_wq_mm(const WqMmArgs* args, const bf16* x, long ldx, const float* 
     if (cudaLaunchKernelEx(&cfg, wq_mm_xprep_kernel, x, ldx, a.m, a.k, ss_in, ss_parts, ss_ld, norm_w, eps, x16) != cudaSuccess)
       return B2_ERR_LAUNCH;
   }
-  const size_t smem = (size_t)a.bufs * 2 * x_sub + (size_t)a.raw_stages * raw + 1024;
+  const size_t smem = (size_t)a.bufs * a.per * 2 * x_sub + (size_t)a.raw_stages * a.per * raw + 1024;
   void (*kern)(const CUtensorMap, const WqMmArgs) = nullptr;
   if (a.bits == 4) kern = a.group == 128 ? wq_mm_kernel<4, 128> : wq_mm_kernel<4, 64>;
   else if (a.bits == 3) kern = a.group == 128 ? wq_mm_kernel<3, 128> : wq_mm_kernel<3, 64>;

@@ -99,3 +99,24 @@ def test_prefill_attention_tiles(T, pos0, hq, hkv, grow):
     ref = torch.einsum("htl,lhd->thd", torch.softmax(s, -1), v.double().repeat_interleave(hq // hkv, 1)).reshape(T, -1)
     assert int(status.item()) == 0
     assert (out.double() - ref).norm() < 6e-3 * ref.norm()
+
+
+# token counts around the padding (16) and the sizes at which the pipeline changes (64 / 65: two units a step or one; 128 /
+# 129: two accumulators or one; 160 / 161: four operand buffers or three); one unit, an odd number of batches, a ragged
+# last row tile, tiles that several CTAs share
+@pytest.mark.parametrize("n,k", [(32, 128), (160, 640), (4128, 384), (256, 2176)])
+@pytest.mark.parametrize("bits,group", [(2, 128), (3, 64), (4, 128)])
+def test_mm_steps(n, k, bits, group):
+    """Against fp64; weights are rounded to fp16 (2^-11) and the result to fp32: below 1e-3 of the norm.  A row's bits do
+    not depend on the rows that travel with it."""
+    lin = L.WqLinear.random(n, k, bits, group, DEV, seed=5)
+    torch.cuda.synchronize()
+    ws = L.GemvWorkspace(DEV)
+    torch.manual_seed(4)
+    x = torch.randn(256, k, device=DEV).to(torch.bfloat16)
+    ref = x.double() @ lin.dequant_cpu().double().to(DEV).t()
+    y = L.mm(lin, x, ws, epi=_lib.EPI_F32)
+    assert (y.double() - ref).norm() < 1e-3 * ref.norm()
+    for m in (1, 16, 17, 64, 65, 128, 129, 160, 161):
+        assert torch.equal(L.mm(lin, x[:m], ws, epi=_lib.EPI_F32), y[:m]), m
+    assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
