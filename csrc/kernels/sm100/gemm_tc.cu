@@ -4,11 +4,14 @@
 // Replaces the reference's cuBLAS path for every prefill GEMM (kernels/src/bf16_linear.cu:54-110, engine call site
 // kernels/m1/m1_model.cu:1875-1895).
 //
-// One CTA computes a 128 x 256 tile.  Warp 0 feeds a 4-stage shared-memory ring with TMA (cp.async.bulk.tensor, 128-byte
+// Persistent: one CTA per SM walks 128 x 256 tiles.  Warp 0 feeds a 4-stage shared-memory ring with TMA (cp.async.bulk.tensor, 128-byte
 // swizzle, every CTA loads its own tiles); one elected thread of warp 1 issues tcgen05.mma (M 128, N 256, K 16 per instruction, operands
-// read through shared-memory descriptors, accumulator = 256 TMEM columns) and commits stage releases and the final
-// "accumulator ready" arrival to mbarriers; warps 2..5 read the accumulator back with tcgen05.ld (each warp owns the
-// 32 TMEM lanes its warp id modulo 4 selects), add the optional residual, convert and store.
+// read through shared-memory descriptors, accumulator = 256 TMEM columns, two of them in turn) and commits stage releases
+// and the "accumulator ready" arrivals to mbarriers; warps 2..5 read the accumulator back with tcgen05.ld (each warp owns
+// the 32 TMEM lanes its warp id modulo 4 selects), add the optional residual, convert and store, while the next tile is
+// being multiplied.  What bounds it: the tensor pipe, 512 cycles per 64 k of a tile at the nominal rate.  With one tile
+// per CTA the set-up, the first loads and the epilogue of every tile were not overlapped: 2048 x
+// 51200 x 5120 781 -> 716 us (1500 TFLOP/s), 2048 x 10240 x 5120 181 -> 165, 1000 x 51200 x 5120 406 -> 368.
 // Every mbarrier wait is bounded; on expiry the CTA records B2_ERR_TIMEOUT, still frees its TMEM and returns.
 #include <cuda.h>
 
@@ -24,7 +27,8 @@ constexpr int A_BYTES = BM * BK * 2;          // 16 KB
 constexpr int B_BYTES = BN * BK * 2;          // 32 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int kGemmThreads = 192;             // 6 warps
-constexpr int kTmemCols = 256;
+constexpr int kTmemCols = 512;               // two accumulators
+constexpr int kSms = 148;
 
 __device__ __forceinline__ void mbar_init_g(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -39,14 +43,22 @@ __device__ __forceinline__ bool mbar_try_wait_g(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait (about two seconds); false = gave up.
+// Bounded wait (about two seconds); false = gave up.  The clock is looked at on every 256th try only.
 __device__ __forceinline__ bool mbar_wait_g(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait_g(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  while (!mbar_try_wait_g(bar, parity)) {
-    if (globaltimer_ns() - t0 > 2000000000ull) return false;
+  uint64_t t0 = 0;
+  for (unsigned it = 1; !mbar_try_wait_g(bar, parity); ++it) {
+    if ((it & 255u) == 0u) {
+      const uint64_t t = globaltimer_ns();
+      if (!t0) t0 = t;
+      else if (t - t0 > 2000000000ull) return false;
+    }
   }
   return true;
+}
+// By a whole warp: the vote brings the lanes back together for what follows and makes the answer uniform.
+__device__ __forceinline__ bool mbar_wait_gw(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_g(bar, parity)) != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
@@ -110,11 +122,11 @@ struct GemmArgs {
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmArgs g) {
   extern __shared__ __align__(1024) uint8_t smem_g[];
-  __shared__ __align__(8) uint64_t full_bar[kStagesG], empty_bar[kStagesG], acc_bar;
+  __shared__ __align__(8) uint64_t full_bar[kStagesG], empty_bar[kStagesG], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_slot;
   __shared__ int s_failed;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // 1024-byte aligned base of the ring (the swizzle pattern is anchored at 1024-byte boundaries)
   const uint32_t ring = (smem_u32(smem_g) + 1023u) & ~1023u;
   // Tile order: groups of up to 16 row tiles sweep the column tiles together, row tile fastest, so that CTAs resident at
@@ -122,16 +134,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   // group instead of once per row tile.
   const int tiles_m = (g.M + BM - 1) / BM, tiles_n = (g.N + BN - 1) / BN;
   constexpr int kGroupM = 16;
-  const int per_group = kGroupM * tiles_n;
-  const int grp = (int)blockIdx.x / per_group;
-  const int gm = min(kGroupM, tiles_m - grp * kGroupM);
-  const int in_grp = (int)blockIdx.x - grp * per_group;
-  const int tile_m = grp * kGroupM + in_grp % gm, tile_n = in_grp / gm;
+  const int per_group = kGroupM * tiles_n, tiles = tiles_m * tiles_n;
+  auto tile_at = [&](int i, int& tm, int& tn) {
+    const int grp = i / per_group, gm = min(kGroupM, tiles_m - grp * kGroupM), in_grp = i - grp * per_group;
+    tn = in_grp / gm;
+    tm = grp * kGroupM + in_grp - tn * gm;
+  };
   const int nkb = (g.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kStagesG; ++i) { mbar_init_g(smem_u32(&full_bar[i]), 1); mbar_init_g(smem_u32(&empty_bar[i]), 1); }
-    mbar_init_g(smem_u32(&acc_bar), 1);
+    for (int i = 0; i < 2; ++i) { mbar_init_g(smem_u32(&acc_full[i]), 1); mbar_init_g(smem_u32(&acc_empty[i]), 4); }
     s_failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -149,48 +162,70 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      for (int kb = 0; kb < nkb; ++kb) {
-        const int s = kb % kStagesG;
-        if (kb >= kStagesG && !mbar_wait_g(smem_u32(&empty_bar[s]), ((kb / kStagesG) - 1) & 1)) { atomicExch(&s_failed, 1); break; }
-        const uint32_t bar = smem_u32(&full_bar[s]);
-        mbar_expect_tx_g(bar, STAGE_BYTES);
-        const uint32_t sa = ring + s * STAGE_BYTES, sb = sa + A_BYTES;
-        tma_load_2d(sa, &map_a, kb * BK, tile_m * BM, bar);
-        tma_load_2d(sb, &map_b, kb * BK, tile_n * BN, bar);
+      int s = 0, n = 0;
+      uint32_t ph = 1;
+      bool ok = true;
+      for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x) {
+        int tile_m, tile_n;
+        tile_at(i, tile_m, tile_n);
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (n >= kStagesG && !mbar_wait_g(smem_u32(&empty_bar[s]), ph)) { ok = false; break; }
+          n += n < kStagesG;
+          const uint32_t bar = smem_u32(&full_bar[s]);
+          mbar_expect_tx_g(bar, STAGE_BYTES);
+          const uint32_t sa = ring + s * STAGE_BYTES, sb = sa + A_BYTES;
+          tma_load_2d(sa, &map_a, kb * BK, tile_m * BM, bar);
+          tma_load_2d(sb, &map_b, kb * BK, tile_n * BN, bar);
+          if (++s == kStagesG) { s = 0; ph ^= 1u; }
+        }
       }
+      if (!ok) atomicExch(&s_failed, 1);
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, BN);
-      bool ok = true;
+    // ---------------- MMA issuer: the whole warp runs the loop, its first lane issues ----------------
+    constexpr uint32_t idesc = make_idesc(BM, BN);
+    int s = 0, t = 0;
+    uint32_t ph = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < tiles && ok; i += gridDim.x, ++t) {
+      const int d = t & 1;
+      const uint32_t td = tmem_base + (uint32_t)(d * BN);
+      if (t >= 2) ok = mbar_wait_gw(smem_u32(&acc_empty[d]), (uint32_t)((t >> 1) - 1) & 1u);
       for (int kb = 0; kb < nkb && ok; ++kb) {
-        const int s = kb % kStagesG;
-        if (!mbar_wait_g(smem_u32(&full_bar[s]), (kb / kStagesG) & 1)) { atomicExch(&s_failed, 1); ok = false; break; }
+        ok = mbar_wait_gw(smem_u32(&full_bar[s]), ph);
+        if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t sa = ring + s * STAGE_BYTES, sb = sa + A_BYTES;
         const uint64_t da = make_desc_sw128(sa), db = make_desc_sw128(sb);
-#pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
+        if (lane == 0) {
           // advancing K by 16 bf16 = 32 bytes inside the 128-byte swizzle atom: +2 in the (>>4) start address field
-          umma_bf16(tmem_base, da + 2 * k, db + 2 * k, idesc, (kb | k) ? 1u : 0u);
+          umma_bf16(td, da, db, idesc, kb ? 1u : 0u);
+#pragma unroll
+          for (int k = 1; k < BK / 16; ++k) umma_bf16(td, da + 2 * k, db + 2 * k, idesc, 1u);
+          umma_commit(smem_u32(&empty_bar[s]));     // frees the stage once these MMAs have read it
+          if (kb == nkb - 1) umma_commit(smem_u32(&acc_full[d]));
         }
-        umma_commit(smem_u32(&empty_bar[s]));     // frees the stage once these MMAs have read it
+        __syncwarp();
+        if (++s == kStagesG) { s = 0; ph ^= 1u; }
       }
-      umma_commit(smem_u32(&acc_bar));            // accumulator complete (arrives even after a failed wait)
     }
+    if (!ok) s_failed = 1;
   } else {
     // ---------------- epilogue: warps 2..5, TMEM lanes 32 * (warp % 4) ----------------
-    const bool ok = mbar_wait_g(smem_u32(&acc_bar), 0);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!ok) atomicExch(&s_failed, 1);
     const int lane_base = (warp & 3) * 32;
-    const int row = tile_m * BM + lane_base + lane;
-    if (ok && !s_failed) {
+    int t = 0;
+    for (int i = blockIdx.x; i < tiles; i += gridDim.x, ++t) {
+      int tile_m, tile_n;
+      tile_at(i, tile_m, tile_n);
+      const int d = t & 1;
+      if (!mbar_wait_gw(smem_u32(&acc_full[d]), (uint32_t)(t >> 1) & 1u)) { s_failed = 1; break; }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tmem_d = tmem_base + (uint32_t)(d * BN);
+      const int row = tile_m * BM + lane_base + lane;
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t r[32];
-        tmem_ld32(tmem_base + ((uint32_t)lane_base << 16) + (uint32_t)c0, r);
+        tmem_ld32(tmem_d + ((uint32_t)lane_base << 16) + (uint32_t)c0, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         const int col = tile_n * BN + c0;
         if (row < g.M && col < g.N) {
@@ -239,12 +274,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
               if (col + i < g.N) *reinterpret_cast<float4*>(fp + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
           }
         }
+        __syncwarp();
       }
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acc_empty[d])) : "memory");
     }
   }
+  __syncwarp();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (threadIdx.x == 0 && s_failed && g.status) atomicExch(g.status, (int)B2_ERR_TIMEOUT);
+  if (s_failed) {
+    if (threadIdx.x == 0 && g.status) atomicExch(g.status, (int)B2_ERR_TIMEOUT);
+    const uint64_t t_end = globaltimer_ns() + 2000000ull;   // copies still in flight get a bounded time to land
+    while (globaltimer_ns() < t_end) { }
+  }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
@@ -305,7 +349,8 @@ static int gemm_launch(const bf16* A, long lda, const bf16* B, long ldb, int M, 
     attr = true;
   }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(((N + BN - 1) / BN) * ((M + BM - 1) / BM), 1, 1);
+  const long tiles = (long)((N + BN - 1) / BN) * ((M + BM - 1) / BM);
+  cfg.gridDim = dim3((unsigned)(tiles < kSms ? tiles : kSms), 1, 1);
   cfg.blockDim = dim3(kGemmThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;

@@ -120,3 +120,17 @@ def test_mm_steps(n, k, bits, group):
     for m in (1, 16, 17, 64, 65, 128, 129, 160, 161):
         assert torch.equal(L.mm(lin, x[:m], ws, epi=_lib.EPI_F32), y[:m]), m
     assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
+
+
+# CTAs that walk one, two and three tiles (148 CTAs; 357 and 162 tiles), ragged rows and columns, fewer k than a stage
+@pytest.mark.parametrize("M,N,K", [(2100, 5128, 128), (257, 13576, 72), (1, 8, 8)])
+def test_gemm_tiles(M, N, K):
+    """Against fp64 in fp32 output: products are exact, sums are fp32 (K roundings of 2^-24)."""
+    from agens_engine_b200.ops import gemm as G
+    torch.manual_seed(M)
+    a, b = torch.randn(M, K, device=DEV).to(torch.bfloat16), torch.randn(N, K, device=DEV).to(torch.bfloat16)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    d = G.gemm_bf16(a, b, out_f32=True, status=status)
+    ref = a.double() @ b.double().t()
+    assert int(status.item()) == 0
+    assert (d.double() - ref).norm() < 1e-5 * ref.norm()
