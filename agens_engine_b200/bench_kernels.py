@@ -181,40 +181,6 @@ def bench_bf16(args):
     print(json.dumps({"peaks": pk, "timing": "CUDA graph of back-to-back launches over rotating weight copies (> L2), median of 10"}))
 
 
-def trace_gemv(args):
-    """Phase stamps of the GEMV on the 32B shapes (m rows), captured inside a CUDA graph of back-to-back launches over
-    rotating weight copies: where the time of one launch goes (start skew, prefetch issue, dependency wait, activation
-    staging, first weights, k loop of the first item, hand-off + epilogue)."""
-    import numpy as np
-    dev = "cuda:0"
-    ws = L.GemvWorkspace(dev, floats=16 << 20)
-    tr = torch.zeros(600 * 8 * 8, dtype=torch.int64, device=dev)
-    L.TRACE_BUFFER = tr
-    shapes = [(10240, 5120), (5120, 8192), (51200, 5120), (5120, 25600)]
-    for n, k in shapes[:1] if args.small else shapes:
-        lin = L.WqLinear.random(n, k, args.bits, 128, dev, seed=1)
-        ncopy = max(4, min(16, (512 << 20) // lin.nbytes() + 1))
-        lins = [L.WqLinear(n, k, args.bits, 128, lin.wq.clone(), lin.ks, lin.rb) for _ in range(ncopy)]
-        x = torch.randn(args.m, k, device=dev).to(torch.bfloat16)
-        out = torch.empty(args.m, n, dtype=torch.bfloat16, device=dev)
-
-        def launch_all():
-            for ln in lins:
-                L.gemv(ln, x, ws, out=out)
-
-        med, _ = graph_time_us(launch_all, len(lins))
-        t = tr.cpu().numpy().reshape(-1, 8)
-        t = t[t[:, 0] > 0]
-        base = t[:, 0].min()
-        q = lambda a: [round(float(np.percentile(a, p)) / 1e3, 2) for p in (0, 50, 100)]
-        print(json.dumps(dict(n=n, k=k, bits=args.bits, m=args.m, ks=lin.ks, rb=lin.rb, us_per_launch=round(med, 2), warps=len(t),
-                              start_skew=q(t[:, 0] - base), prefetch_issue=q(t[:, 1] - t[:, 0]), dependency_wait=q(t[:, 2] - t[:, 1]),
-                              activation_staging=q(t[:, 3] - t[:, 2]), first_weights=q(t[:, 4] - t[:, 3]),
-                              k_loop_first_item=q(t[:, 5] - t[:, 3]), handoff_epilogue=q(t[:, 6] - t[:, 5]),
-                              end=q(t[:, 6] - base), unit="us [min, median, max] over warps of the last launch")), flush=True)
-    L.TRACE_BUFFER = None
-
-
 def bench_mm(args):
     """Mixed-bit tcgen05 GEMM (in-kernel dequantisation) on the 32B shapes for m rows, CUDA-graph timing over rotating
     weight copies larger than L2."""
@@ -410,7 +376,7 @@ def profile_step(args):
 
 def main(argv=None):
     ap = argparse.ArgumentParser()
-    ap.add_argument("what", choices=["gemv", "bf16", "attn", "gemm", "profile_gemv", "trace_gemv", "mm", "profile_mm", "profile_attn", "profile_attn_tc", "profile_gemm", "profile_misc", "profile_step"])
+    ap.add_argument("what", choices=["gemv", "bf16", "attn", "gemm", "profile_gemv", "mm", "profile_mm", "profile_attn", "profile_attn_tc", "profile_gemm", "profile_misc", "profile_step"])
     ap.add_argument("--layers", type=int, default=0)
     ap.add_argument("--bits", type=int, default=4)
     ap.add_argument("--ks", type=int, default=0)
@@ -427,8 +393,6 @@ def main(argv=None):
         profile_gemv(args)
     elif args.what == "gemm":
         bench_gemm(args)
-    elif args.what == "trace_gemv":
-        trace_gemv(args)
     elif args.what == "mm":
         bench_mm(args)
     elif args.what == "profile_mm":

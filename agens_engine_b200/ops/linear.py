@@ -1,6 +1,7 @@
 """Quantised linears on the GPU: FM weight holder + GEMV launcher (decode / verify / small batch).
 
-Python here only assembles argument blocks; the arithmetic is in ``csrc/kernels/sm100/wq_gemv.cu``.
+Python here only assembles argument blocks; the arithmetic is in ``csrc/kernels/sm100/wq_gemv8.cu`` (one to eight rows, more
+in chunks of eight), ``wq_mm.cu`` (tensor-core GEMM) and ``wq_gemv.cu`` (the tensor-parallel push epilogue).
 """
 from __future__ import annotations
 
@@ -215,8 +216,8 @@ class GemvWorkspace:
 
 
 MM_MIN_ROWS = int(os.environ.get("B200E_MM_MIN_ROWS", "9"))     # token rows from which the tcgen05 GEMM takes over
-# Measurement aids.  Only a library built with B200E_NVCC_DEFS=-DB2_MEASURE reads these fields; the production kernels
-# have the modes compiled out, so a stray environment variable cannot change results.
+# Measurement aids of the push-epilogue GEMV (wq_gemv.cu).  Only a library built with B200E_NVCC_DEFS=-DB2_MEASURE reads
+# these fields; the production kernels have the modes compiled out, so a stray environment variable cannot change results.
 TRACE_BUFFER = None      # int64 CUDA tensor [CTAs * 8 warps * 8] that receives the GEMV's phase stamps
 GEMV_DEBUG = int(os.environ.get("B200E_GEMV_DEBUG", "0"))
 
