@@ -51,9 +51,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after about two seconds and reports failure instead of hanging the GPU.  The clock is looked at
-// on every 256th try only: reading it takes longer than a try.
+// Bounded wait: gives up after about two seconds and reports failure instead of hanging the GPU.
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const uint64_t t0 = globaltimer_ns();
+  while (!mbar_try_wait(bar, parity)) {
+    if (globaltimer_ns() - t0 > 2000000000ull) return false;
+  }
+  return true;
+}
+// The same, looking at the clock on every 256th try only, for loops that wait often.
+__device__ __forceinline__ bool mbar_wait_quick(uint32_t bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;
   uint64_t t0 = 0;
   for (unsigned it = 1; !mbar_try_wait(bar, parity); ++it) {

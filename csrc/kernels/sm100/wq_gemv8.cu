@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kT8, 1) wq_gemv8_kernel(const WqGemvArgs a, co
 #pragma unroll 1
     for (int i = 0; i < cnt; ++i) {
       if (!mbar_try_wait(cbar, cph)) {            // the lanes come back together before the .aligned mma
-        if (!__all_sync(0xffffffffu, mbar_wait_bounded(cbar, cph))) {
+        if (!__all_sync(0xffffffffu, mbar_wait_quick(cbar, cph))) {
           if (a.status && lane == 0) atomicExch(a.status, (int)B2_ERR_TIMEOUT);
           failed = true;
           break;

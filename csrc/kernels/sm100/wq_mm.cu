@@ -62,10 +62,10 @@ constexpr int kTmemColsM = 512;
 __device__ __forceinline__ void mbar_arrive_m(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// mbar_wait_bounded by a whole warp: its lanes may leave the wait at different tries, and the tcgen05.ld and .st that follow are
+// mbar_wait_quick by a whole warp: its lanes may leave the wait at different tries, and the tcgen05.ld and .st that follow are
 // .aligned; the vote brings the lanes back together and makes the answer uniform.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity)) != 0;
+  return __all_sync(0xffffffffu, mbar_wait_quick(bar, parity)) != 0;
 }
 __device__ __forceinline__ void tma_load_2d_m(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
       RingPos r;
       for (int i = 0, st = 0; i < nu; ++st, r.next(NB)) {
         const int cnt = min(P, min(nbat - kb, nu - i));
-        if (st >= NB && !mbar_wait_bounded(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
+        if (st >= NB && !mbar_wait_quick(smem_u32(&op_empty[r.s]), r.ph ^ 1u)) { atomicExch(&s_failed, 1); break; }
         const uint32_t bar = smem_u32(&op_full[r.s]);
         mbar_expect_tx(bar, (uint32_t)cnt * 2 * x_sub);
         for (int h = 0; h < 2 * cnt; ++h) tma_load_2d_m(x_ring + r.s * x_step + h * x_sub, &map_x, kb * 128 + h * BKS, 0, bar);
