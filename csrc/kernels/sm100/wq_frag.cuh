@@ -73,6 +73,11 @@ __device__ __forceinline__ bool mbar_wait_quick(uint32_t bar, uint32_t parity) {
   }
   return true;
 }
+// mbar_wait_quick by a whole warp.  Lanes may leave a wait at different tries; the vote, which every lane reaches whatever
+// its own try said, brings them back together for the .aligned instructions that follow and makes the answer uniform.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_quick(bar, parity)) != 0;
+}
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");

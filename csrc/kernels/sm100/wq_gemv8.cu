@@ -337,14 +337,11 @@ __global__ void __launch_bounds__(kT8, 1) wq_gemv8_kernel(const WqGemvArgs a, co
       for (int i = 0; i < 4; ++i) y[r][i] = 0.f;
 #pragma unroll 1
     for (int i = 0; i < cnt; ++i) {
-      if (!mbar_try_wait(cbar, cph)) {            // the lanes come back together before the .aligned mma
-        if (!__all_sync(0xffffffffu, mbar_wait_quick(cbar, cph))) {
-          if (a.status && lane == 0) atomicExch(a.status, (int)B2_ERR_TIMEOUT);
-          failed = true;
-          break;
-        }
+      if (!mbar_wait_warp(cbar, cph)) {           // voted: the mma below are .aligned
+        if (a.status && lane == 0) atomicExch(a.status, (int)B2_ERR_TIMEOUT);
+        failed = true;
+        break;
       }
-      __syncwarp();
       WFrag<BITS, GROUP> cf[2];
 #pragma unroll
       for (int r = 0; r < 2; ++r)
@@ -391,6 +388,7 @@ __global__ void __launch_bounds__(kT8, 1) wq_gemv8_kernel(const WqGemvArgs a, co
       if (cbar == bars_u + NST * 8) { cbar = bars_u; cptr = ring; cph ^= 1u; }
       __syncwarp();                               // the stage is free again
       if (lane == 0 && pleft > 0) issue();
+      __syncwarp();
     }
     if (failed) break;
     // fragment layout -> tile [tok][32 rows]; the first fragment of a warp has its own tile, the others use the second

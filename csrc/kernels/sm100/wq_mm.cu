@@ -62,11 +62,6 @@ constexpr int kTmemColsM = 512;
 __device__ __forceinline__ void mbar_arrive_m(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// mbar_wait_quick by a whole warp: its lanes may leave the wait at different tries, and the tcgen05.ld and .st that follow are
-// .aligned; the vote brings the lanes back together and makes the answer uniform.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, mbar_wait_quick(bar, parity)) != 0;
-}
 __device__ __forceinline__ void tma_load_2d_m(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

@@ -1,0 +1,45 @@
+"""Warp-wide instructions of the kernels, checked on their sources: undefined behaviour of this kind (a full-mask vote or an
+``.aligned`` instruction that some lanes of a warp do not execute) cannot be provoked safely on a GPU."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "csrc"
+SOURCES = sorted(list((CSRC / "kernels").rglob("*.cu")) + list((CSRC / "kernels").rglob("*.cuh")))
+# every wait on an mbarrier whose answer is a lane's own
+LANE_WAIT = re.compile(r"\b(\w*mbar_try\w*|mbar_wait_bounded|mbar_wait_quick|mbar_wait_g)\s*\(")
+WARP_WIDE = re.compile(r"\b__(all|any|ballot|shfl\w*|match\w*|reduce\w*)_sync\s*\(|\b__syncwarp\s*\(|\.aligned")
+
+
+def _code(path):
+    """The source without comments, positions kept."""
+    blank = lambda m: re.sub(r"[^\n]", " ", m.group(0))
+    return re.sub(r"//[^\n]*|/\*.*?\*/", blank, path.read_text(), flags=re.S)
+
+
+def _close(s, i, pair):
+    """Position after the bracket that closes the one at s[i]."""
+    depth = 0
+    for j in range(i, len(s)):
+        depth += (s[j] == pair[0]) - (s[j] == pair[1])
+        if depth == 0:
+            return j + 1
+    raise AssertionError("unbalanced")
+
+
+def _branches(s):
+    """(condition, body, line) of every if / while / for."""
+    for m in re.finditer(r"\b(if|while|for)\s*\(", s):
+        end = _close(s, m.end() - 1, "()")
+        b = re.compile(r"\s*").match(s, end).end()
+        body = s[b:_close(s, b, "{}")] if s[b] == "{" else s[b:s.index(";", b) + 1]
+        yield s[m.end():end - 1], body, s.count("\n", 0, m.start()) + 1
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_no_warp_wide_instruction_under_a_lanes_own_wait(path):
+    """A branch on a lane's own wait, taken by some lanes and not by others, holds nothing that all lanes have to execute."""
+    bad = [(line, cond.strip()) for cond, body, line in _branches(_code(path))
+           if LANE_WAIT.search(re.sub(r"__all_sync\s*\([^;]*", "", cond)) and WARP_WIDE.search(body)]
+    assert not bad, bad
