@@ -411,6 +411,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             if (c0 + j < t1) mine[(size_t)(c0 + j) * BM] = __uint_as_float(r[j]);
+          __syncwarp();
         }
         __threadfence();
         c_first = (int)((((long)tile * nbat + 1) * a.ctas - 1) / U);
@@ -460,6 +461,7 @@ __global__ void __launch_bounds__(kMmThreads, 1) wq_mm_kernel(const __grid_const
             case EPI_F32: mm_emit16<EPI_F32>(a, v, c0, t1, row, row_ok, part, npan, lane); break;
             default: mm_emit16<EPI_ARGMAX>(a, v, c0, t1, row, row_ok, part, npan, lane); break;
           }
+          __syncwarp();                                   // single lanes store in there; the next tcgen05.ld is .aligned
         }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -43,3 +43,23 @@ def test_no_warp_wide_instruction_under_a_lanes_own_wait(path):
     bad = [(line, cond.strip()) for cond, body, line in _branches(_code(path))
            if LANE_WAIT.search(re.sub(r"__all_sync\s*\([^;]*", "", cond)) and WARP_WIDE.search(body)]
     assert not bad, bad
+
+
+def _loops(s):
+    """(body, line) of every for loop."""
+    for m in re.finditer(r"\bfor\s*\(", s):
+        b = re.compile(r"\s*").match(s, _close(s, m.end() - 1, "()")).end()
+        if s[b] == "{":
+            yield s[b:_close(s, b, "{}")], s.count("\n", 0, m.start()) + 1
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_loops_over_tensor_memory_bring_the_warp_together(path):
+    """A loop that reads TMEM (tcgen05.ld is .aligned) and writes results with the lanes on their own also has a
+    __syncwarp, so that every turn starts with the whole warp."""
+    s = _code(path)
+    readers = re.findall(r"\bvoid\s+(\w+)\(.*\{\s*asm volatile\(\s*\"tcgen05\.ld", s)
+    assert bool(readers) == ("tcgen05.ld" in s)
+    bad = [line for body, line in _loops(s)
+           if any(re.search(r"\b%s\s*\(" % r, body) for r in readers) and re.search(r"\bif\b", body) and "__syncwarp" not in body]
+    assert not bad, bad
