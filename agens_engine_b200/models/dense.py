@@ -164,7 +164,7 @@ class DenseModel:
         """Size the split-k workspace from the loaded linears (call once after the weights are in place)."""
         lib = _lib.cuda_lib()
         lins = [x for x in [self.lm_head] + [d[lin] for d in self.layers for lin in LINEARS] if isinstance(x, L.WqLinear)]
-        need = max(lib.b2_wq_gemv_scratch_floats(x.n, x.k, x.ks, r, M_GEMV) for x in lins for r in (2, x.rb))
+        need = max(L.gemv_scratch_floats(x, M_GEMV) for x in lins)
         # the tensor-core path's split-k partials at its largest row count, so that the scratch never moves afterwards
         need = max(need, max(lib.b2_wq_mm_scratch_floats(x.n, x.k, 256) for x in lins))
         panels = max(x.n_panels() for x in lins)

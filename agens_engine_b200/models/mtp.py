@@ -95,8 +95,7 @@ class MtpHead(DenseModel):
     def finalize(self):
         super().finalize()
         if self.fc is not None:
-            from .. import _lib
-            need = _lib.cuda_lib().b2_wq_gemv_scratch_floats(self.fc.n, self.fc.k, self.fc.ks, 2, M_GEMV)
+            need = L.gemv_scratch_floats(self.fc, M_GEMV)
             if need > self.ws.scratch.numel():
                 self.ws = L.GemvWorkspace(self.dev, floats=need, panels=max(self.ws.counters.numel(), 1 << 10))
         return self

@@ -191,6 +191,13 @@ def _bf16_linear(lin: Bf16Linear, x: torch.Tensor, *, epi: int, pro: int, norm_w
     raise ValueError("this epilogue is not available for a bf16 linear (the lm_head is quantised at load)")
 
 
+def gemv_scratch_floats(lin: WqLinear, m: int) -> int:
+    """Scratch that :func:`gemv` wants for up to ``m`` rows of this linear, with and without the push epilogue."""
+    lib = _lib.cuda_lib()
+    return max(lib.b2_wq_gemv8_scratch_floats(lin.n, lin.k, m),
+               *(lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, rb, m) for rb in (2, lin.rb)))
+
+
 class GemvWorkspace:
     """Split-k scratch, self-resetting item counters and the status word shared by the GEMV / GEMM launches of one
     stream, plus the fp16 activation staging buffer of the tensor-core path (grown on first use)."""

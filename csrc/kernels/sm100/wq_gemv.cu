@@ -576,11 +576,10 @@ B2_API int b2_wq_gemv_fmax(int n, int k, int ks, int rb) {
   const long per = U / V;                       // every worker owns per or per + 1 units
   return (int)((nb + per - 1) / per + 1);
 }
-// Scratch floats for the split partials: [item][ks][fmax][m][rows per item], and no less than b2_wq_gemv8 needs.
+// Scratch floats for the split partials: [item][ks][fmax][m][rows per item].
 B2_API long b2_wq_gemv_scratch_floats(int n, int k, int ks, int rb, int m) {
   const long nitems = (n / 32 + rb / 2 - 1) / (rb / 2);
-  const long here = nitems * ks * b2_wq_gemv_fmax(n, k, ks, rb) * (long)m * rb * 16, other = b2_wq_gemv8_scratch_floats(n, k, m);
-  return here > other ? here : other;
+  return nitems * ks * b2_wq_gemv_fmax(n, k, ks, rb) * (long)m * rb * 16;
 }
 
 // Launches the GEMV described by *args on `stream`.  Returns a b2::Status; nothing is launched on B2_ERR_ARG.

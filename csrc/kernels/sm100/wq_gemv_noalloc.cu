@@ -87,8 +87,21 @@ extern "C" int b2_wq_gemv_noalloc(const uint8_t* wq, int n, int k, int bits, int
   a.scratch = s->partials;
   a.counters = s->counters;
   a.status = s->status;
-  // the kernel of the regular entry point, unless its scratch exceeds the array where the other's does not
-  const int st = b2_wq_gemv8_scratch_floats(n, k, m) <= (long)B2_NOALLOC_SCRATCH_FLOATS ? b2_wq_gemv8(&a, stream) : b2_wq_gemv(&a, stream);
+  // The kernel of the regular entry point.  Which problems are accepted is b2_wq_gemv's scratch, above; b2_wq_gemv8 hands
+  // panels over per slice and CTA and may want more for the same rows, so it takes as many rows at a time as the array
+  // holds (a row's bits do not depend on the rows that travel with it).  Where not even one fits, a matter of (n, k) only,
+  // b2_wq_gemv runs.
+  int rows = 8;
+  while (rows > 0 && b2_wq_gemv8_scratch_floats(n, k, rows) > (long)B2_NOALLOC_SCRATCH_FLOATS) rows /= 2;
+  int st = 0;
+  if (rows == 0) st = b2_wq_gemv(&a, stream);
+  for (int t0 = 0; rows > 0 && t0 < m && st == 0; t0 += rows) {
+    b2::WqGemvArgs c = a;
+    c.m = m - t0 < rows ? m - t0 : rows;
+    c.x += (long)t0 * ldx;
+    c.y += (long)t0 * ldy;
+    st = b2_wq_gemv8(&c, stream);
+  }
   if (st != 0) {
     set_err(err, st == 1 ? "b2_wq_gemv_noalloc: the GEMV launcher rejected the arguments (alignment of x / ldx?)"
                          : "b2_wq_gemv_noalloc: kernel launch failed");

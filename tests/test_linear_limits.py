@@ -1,0 +1,61 @@
+"""Which calls of the quantised linears are accepted: host-side rules, read without a GPU."""
+import ctypes as C
+
+import pytest
+import torch
+
+from agens_engine_b200 import _lib
+
+needs_no_gpu = pytest.mark.skipif(torch.cuda.is_available(), reason="the accepted calls would run on made-up addresses")
+
+
+# (n, k, slices of k, rows): accepted by the limit in wq_gemv_noalloc.h, 2^20 scratch floats of the kernel with slices
+FITS = [(40960, 8192, 1, 8), (151936, 6144, 1, 3), (151936, 8192, 1, 2), (57344, 8192, 1, 5), (11040, 28672, 2, 8), (256, 2048, 4, 3)]
+TOO_LARGE = [(151936, 5120, 2, 32), (40960, 8192, 1, 16), (262176, 128, 1, 1)]
+
+
+@needs_no_gpu
+@pytest.mark.parametrize("n,k,ks,m,fits", [s + (True,) for s in FITS] + [s + (False,) for s in TOO_LARGE])
+def test_allocation_free_gemv_accepts_what_its_header_says(n, k, ks, m, fits):
+    """A refusal is 1 and launches nothing; an accepted call goes on to the device, which is not there (2)."""
+    lib = _lib.cuda_lib()
+    need = lib.b2_wq_gemv_scratch_floats(n, k, ks, 2, m)
+    assert (need <= 1 << 20 and n // 32 <= 8192) == fits
+    err = C.create_string_buffer(160)
+    fn = lib.b2_wq_gemv_noalloc
+    fn.argtypes = [C.c_void_p] + [C.c_int] * 5 + [C.c_void_p, C.c_long, C.c_int, C.c_void_p, C.c_long, C.c_void_p, C.c_void_p, C.c_char_p]
+    fn.restype = C.c_int
+    rc = fn(256, n, k, 4, 128, ks, 256, k, m, 256, n, None, None, err)
+    assert rc == (2 if fits else 1), err.value
+
+
+def _panel_reference(lin, x, panels):
+    """fp64 results of some 32-row panels, from their packed bytes."""
+    from agens_engine_b200.ops import linear as L
+    size = L.fm_bytes(32, lin.k, lin.bits, lin.group)
+    w = torch.cat([L.WqLinear(32, lin.k, lin.bits, lin.group, lin.wq[p * size:(p + 1) * size]).dequant_cpu() for p in panels])
+    return x.double() @ w.double().to(x.device).t(), torch.cat([torch.arange(32 * p, 32 * p + 32) for p in panels])
+
+
+# all rows at once, fewer rows at a time than asked for, and a shape of which not one row fits the newer kernel's scratch
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k,ks,m,bits", [(57344, 8192, 1, 3, 2), (40960, 8192, 1, 8, 4), (11040, 28672, 2, 7, 3), (40960, 81920, 4, 3, 2)])
+def test_allocation_free_gemv_near_its_limit(n, k, ks, m, bits):
+    """bf16 result of fp16 activations: two roundings of 2^-9 and 2^-11 relative to the norm, below 4e-3."""
+    from agens_engine_b200.ops import linear as L
+    lib = _lib.cuda_lib()
+    fn = lib.b2_wq_gemv_noalloc
+    fn.argtypes = [C.c_void_p] + [C.c_int] * 5 + [C.c_void_p, C.c_long, C.c_int, C.c_void_p, C.c_long, C.c_void_p, C.c_void_p, C.c_char_p]
+    fn.restype = C.c_int
+    lin = L.WqLinear.random(n, k, bits, 128, "cuda:0", seed=n, ks=ks)
+    x = torch.randn(m, k, device="cuda:0").to(torch.bfloat16)
+    y = torch.full((m, n), float("nan"), dtype=torch.bfloat16, device="cuda:0")
+    status, err = torch.full((1,), -1, dtype=torch.int32, device="cuda:0"), C.create_string_buffer(160)
+    rc = fn(lin.wq.data_ptr(), n, k, bits, 128, ks, x.data_ptr(), k, m, y.data_ptr(), n, status.data_ptr(), _lib.current_stream(), err)
+    assert rc == 0, err.value
+    assert int(status.item()) == 0 and bool(torch.isfinite(y).all())
+    ref, rows = _panel_reference(lin, x, [0, 1, n // 64, n // 32 - 1])
+    assert (y[:, rows].double() - ref).norm() < 4e-3 * ref.norm()
+    one = torch.full((1, n), float("nan"), dtype=torch.bfloat16, device="cuda:0")       # a row's bits do not depend on its company
+    assert fn(lin.wq.data_ptr(), n, k, bits, 128, ks, x[m - 1].data_ptr(), k, 1, one.data_ptr(), n, None, _lib.current_stream(), err) == 0
+    assert torch.equal(one[0], y[m - 1])
