@@ -207,6 +207,7 @@ class GemvWorkspace:
         self.counters = torch.zeros(panels, dtype=torch.int32, device=device)
         # the status word may live inside a block of status words that the owner reads with one copy
         self.status = status if status is not None else torch.zeros(1, dtype=torch.int32, device=device)
+        self._outgrown = []
         self.x16 = None
         self.mm_min_rows = None      # overrides MM_MIN_ROWS for the launches that use this workspace
 
@@ -218,7 +219,10 @@ class GemvWorkspace:
         return self.x16
 
     def ensure_scratch(self, floats: int):
+        """A larger linear than the workspace was sized for makes the scratch grow.  What it replaces is kept: CUDA graphs
+        captured before go on using that memory."""
         if floats > self.scratch.numel():
+            self._outgrown.append(self.scratch)
             self.scratch = torch.empty(floats, dtype=torch.float32, device=self.scratch.device)
 
 
@@ -279,7 +283,6 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
     if resid is not None:
         a.resid, a.ldr = ptr(resid), resid.stride(0)
     a.ss_out = ptr(ss_out)
-    a.scratch, a.counters = ptr(ws.scratch), ptr(ws.counters)
     a.status = ptr(ws.status)
     if tp is None:
         need = lib.b2_wq_gemv8_scratch_floats(lin.n, lin.k, m)
@@ -288,8 +291,10 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
         a.fmax = lib.b2_wq_gemv_fmax(lin.n, lin.k, lin.ks, a.rb)
         a.debug, a.trace, a.tp = GEMV_DEBUG, ptr(TRACE_BUFFER), tp
         need = lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, a.rb, m)
-    if need > ws.scratch.numel() or lin.n_panels() > ws.counters.numel():
-        raise RuntimeError(f"GEMV workspace too small: need {need} floats, {lin.n_panels()} counters")
+    if lin.n_panels() > ws.counters.numel():
+        raise RuntimeError(f"GEMV workspace too small: need {lin.n_panels()} counters")
+    ws.ensure_scratch(need)
+    a.scratch, a.counters = ptr(ws.scratch), ptr(ws.counters)
     with torch.cuda.device(dev):
         if tp is None:
             check(lib.b2_wq_gemv8(C.byref(a), current_stream()), "b2_wq_gemv8")

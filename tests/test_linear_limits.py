@@ -59,3 +59,28 @@ def test_allocation_free_gemv_near_its_limit(n, k, ks, m, bits):
     one = torch.full((1, n), float("nan"), dtype=torch.bfloat16, device="cuda:0")       # a row's bits do not depend on its company
     assert fn(lin.wq.data_ptr(), n, k, bits, 128, ks, x[m - 1].data_ptr(), k, 1, one.data_ptr(), n, None, _lib.current_stream(), err) == 0
     assert torch.equal(one[0], y[m - 1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,k,floats", [(151936, 5248, 4 << 20), (2048, 5248, 1 << 10)])
+def test_gemv_grows_its_workspace(n, k, floats):
+    """Slices of k (above 5120 inputs) hand every panel over through scratch; a workspace that is too small for that
+    grows, and a graph captured before keeps its own."""
+    from agens_engine_b200.ops import linear as L
+    lin, small = L.WqLinear.random(n, k, 4, 128, "cuda:0", seed=n), L.WqLinear.random(64, 512, 4, 128, "cuda:0", seed=1)
+    ws = L.GemvWorkspace("cuda:0", floats=floats)
+    x, xs = torch.randn(8, k, device="cuda:0").to(torch.bfloat16), torch.randn(2, 512, device="cuda:0").to(torch.bfloat16)
+    ys = L.gemv(small, xs, ws, epi=_lib.EPI_F32)
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        L.gemv(small, xs, ws, epi=_lib.EPI_F32, out=ys)
+    y = L.gemv(lin, x, ws, epi=_lib.EPI_F32)
+    assert ws.scratch.numel() > floats
+    ref, rows = _panel_reference(lin, x, [0, n // 64, n // 32 - 1])
+    assert (y[:, rows].double() - ref).norm() < 1e-3 * ref.norm()
+    want = ys.clone()
+    ys.zero_()
+    graph.replay()
+    assert torch.equal(ys, want) and torch.equal(L.gemv(lin, x, ws, epi=_lib.EPI_F32), y)
+    assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
