@@ -171,6 +171,7 @@ def _declare(lib: C.CDLL):
     sig = {
         "b2_wq_gemv": ([C.POINTER(WqGemvArgs), vp], i),
         "b2_wq_gemv8": ([C.POINTER(WqGemvArgs), vp], i), "b2_wq_gemv8_scratch_floats": ([i, i, i], l),
+        "b2_wq_gemv8_takes": ([i, i], i),
         "b2_wq_gemv_scratch_floats": ([i, i, i, i, i], l),
         "b2_wq_gemv_vworkers": ([i, i, i, i], i),
         "b2_wq_gemv_fmax": ([i, i, i, i], i),

@@ -284,22 +284,26 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
         a.resid, a.ldr = ptr(resid), resid.stride(0)
     a.ss_out = ptr(ss_out)
     a.status = ptr(ws.status)
-    if tp is None:
+    # the push all-reduce epilogue, and matrices beyond the other kernel's schedule, run on the kernel with k slices
+    old = tp is not None or not lib.b2_wq_gemv8_takes(lin.n, lin.k)
+    if not old:
         need = lib.b2_wq_gemv8_scratch_floats(lin.n, lin.k, m)
     else:
         a.vworkers = lib.b2_wq_gemv_vworkers(lin.n, lin.k, lin.ks, a.rb)
         a.fmax = lib.b2_wq_gemv_fmax(lin.n, lin.k, lin.ks, a.rb)
-        a.debug, a.trace, a.tp = GEMV_DEBUG, ptr(TRACE_BUFFER), tp
+        a.debug, a.trace = GEMV_DEBUG, ptr(TRACE_BUFFER)
+        if tp is not None:
+            a.tp = tp
         need = lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, a.rb, m)
     if lin.n_panels() > ws.counters.numel():
         raise RuntimeError(f"GEMV workspace too small: need {lin.n_panels()} counters")
     ws.ensure_scratch(need)
     a.scratch, a.counters = ptr(ws.scratch), ptr(ws.counters)
     with torch.cuda.device(dev):
-        if tp is None:
-            check(lib.b2_wq_gemv8(C.byref(a), current_stream()), "b2_wq_gemv8")
-        else:                                   # the push all-reduce epilogue is in the other kernel of the family
+        if old:
             check(lib.b2_wq_gemv(C.byref(a), current_stream()), "b2_wq_gemv")
+        else:
+            check(lib.b2_wq_gemv8(C.byref(a), current_stream()), "b2_wq_gemv8")
     return out
 
 

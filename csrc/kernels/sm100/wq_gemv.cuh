@@ -67,6 +67,7 @@ B2_API int b2_wq_gemv_vworkers(int n, int k, int ks, int rb);
 B2_API int b2_wq_gemv_fmax(int n, int k, int ks, int rb);
 B2_API long b2_wq_gemv_scratch_floats(int n, int k, int ks, int rb, int m);
 B2_API int b2_wq_gemv8(const b2::WqGemvArgs* args, cudaStream_t stream);
+B2_API int b2_wq_gemv8_takes(int n, int k);
 B2_API long b2_wq_gemv8_scratch_floats(int n, int k, int m);
 B2_API long b2_wq_bytes(int n, int k, int bits, int group);
 B2_API int b2_wq_dequant(const uint8_t* wq, int n, int k, int bits, int group, bf16* out, long ldo, cudaStream_t stream);

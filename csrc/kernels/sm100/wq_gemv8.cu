@@ -488,6 +488,12 @@ B2_API long b2_wq_gemv8_scratch_floats(int n, int k, int m) {
   return (long)p.slices * (n / 32) * p.fmax * (m < 8 ? m : 8) * 32;
 }
 
+// Whether b2_wq_gemv8 takes a matrix: unit numbers times CTAs fit 32 bits, and the hand-over has a lane for every slice
+// (k up to 163840).  b2_wq_gemv has neither limit there.  A matter of (n, k) only.
+B2_API int b2_wq_gemv8_takes(int n, int k) {
+  return (double)(n / 32) * (double)(k / 128) * 148.0 < 4.0e9 && g8_plan(n, k).slices <= 32;
+}
+
 // The GEMV of *args (fields vworkers, fmax and tp are not read, ks and rb do not matter) for 1 .. 32 rows, eight at a time.  `counters`
 // holds n / 32 self-resetting words, `scratch` b2_wq_gemv8_scratch_floats(n, k, m) floats.
 B2_API int b2_wq_gemv8(const WqGemvArgs* args, cudaStream_t stream) {
@@ -497,9 +503,8 @@ B2_API int b2_wq_gemv8(const WqGemvArgs* args, cudaStream_t stream) {
   if (a.ks < 1 || a.ks > kMaxKs || a.k / 128 % a.ks || (a.rb != 2 && a.rb != 4)) return B2_ERR_ARG;   // a linear that the other kernel takes
   if (!a.scratch || !a.counters || a.epi == EPI_TP_RESID) return B2_ERR_ARG;
   if ((a.ldx % 8) || (reinterpret_cast<uintptr_t>(a.x) & 15)) return B2_ERR_ARG;
-  if ((double)(a.n / 32) * (double)(a.k / 128) * 148.0 >= 4.0e9) return B2_ERR_ARG;   // 32-bit schedule arithmetic
+  if (!b2_wq_gemv8_takes(a.n, a.k)) return B2_ERR_ARG;
   const Gemv8Plan p = g8_plan(a.n, a.k);
-  if (p.slices > 32) return B2_ERR_ARG;
   for (int t0 = 0; t0 < a.m; t0 += 8) {
     WqGemvArgs c = a;
     c.m = a.m - t0 < 8 ? a.m - t0 : 8;

@@ -89,9 +89,9 @@ extern "C" int b2_wq_gemv_noalloc(const uint8_t* wq, int n, int k, int bits, int
   a.status = s->status;
   // The kernel of the regular entry point.  Which problems are accepted is b2_wq_gemv's scratch, above; b2_wq_gemv8 hands
   // panels over per slice and CTA and may want more for the same rows, so it takes as many rows at a time as the array
-  // holds (a row's bits do not depend on the rows that travel with it).  Where not even one fits, a matter of (n, k) only,
-  // b2_wq_gemv runs.
-  int rows = 8;
+  // holds (a row's bits do not depend on the rows that travel with it).  Where not even one fits, or the matrix is not one
+  // that it takes, both a matter of (n, k) only, b2_wq_gemv runs.
+  int rows = b2_wq_gemv8_takes(n, k) ? 8 : 0;
   while (rows > 0 && b2_wq_gemv8_scratch_floats(n, k, rows) > (long)B2_NOALLOC_SCRATCH_FLOATS) rows /= 2;
   int st = 0;
   if (rows == 0) st = b2_wq_gemv(&a, stream);

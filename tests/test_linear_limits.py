@@ -84,3 +84,20 @@ def test_gemv_grows_its_workspace(n, k, floats):
     graph.replay()
     assert torch.equal(ys, want) and torch.equal(L.gemv(lin, x, ws, epi=_lib.EPI_F32), y)
     assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bits", [2, 4])
+def test_gemv_of_very_many_inputs(bits):
+    """33 slices of k, one more than the hand-over of the kernel for one to eight rows has lanes."""
+    from agens_engine_b200.ops import linear as L
+    n, k = 96, 164352
+    assert not _lib.cuda_lib().b2_wq_gemv8_takes(n, k) and _lib.cuda_lib().b2_wq_gemv8_takes(n, 163840)
+    lin = L.WqLinear.random(n, k, bits, 128, "cuda:0", seed=9)
+    x = torch.randn(5, k, device="cuda:0").to(torch.bfloat16)
+    ws = L.GemvWorkspace("cuda:0")
+    y = L.gemv(lin, x, ws, epi=_lib.EPI_F32)
+    ref, rows = _panel_reference(lin, x, [0, 1, 2])
+    assert (y[:, rows].double() - ref).norm() < 1e-3 * ref.norm()
+    assert torch.equal(L.gemv(lin, x[3:4], ws, epi=_lib.EPI_F32)[0], y[3])
+    assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
