@@ -108,32 +108,22 @@ __global__ void __launch_bounds__(kT8, 1) wq_gemv8_kernel(const WqGemvArgs a, co
     for (int i = 0; i < NST && pleft > 0; ++i) issue();
   }
   __syncwarp();
-  // the norm weights of this thread's first two items, too
   const int nvec = len * 16, total = nvec * m;
   auto item = [&](int i, int& tok, int& v) { tok = ONE ? 0 : i / nvec; v = i - tok * nvec; };
   uint4 pre[2], prw[2];
-#pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const int i = (int)threadIdx.x + j * kT8;
-    prw[j] = make_uint4(0u, 0u, 0u, 0u);
-    if (a.pro == PRO_NORM && i < total) {
-      int tok, v;
-      item(i, tok, v);
-      prw[j] = *reinterpret_cast<const uint4*>(a.norm_w + base * 128 + v * 8);
-    }
-  }
-  pdl_wait();
+  pdl_wait();                      // nothing but packed weights is read before this
   pdl_launch_dependents();
 
   // ---- stage the activations of the slice: fp16(x / c) and the per-group sums ----
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int i = (int)threadIdx.x + j * kT8;
-    pre[j] = make_uint4(0u, 0u, 0u, 0u);
+    pre[j] = prw[j] = make_uint4(0u, 0u, 0u, 0u);
     if (i < total) {
       int tok, v;
       item(i, tok, v);
       pre[j] = *reinterpret_cast<const uint4*>(a.x + (size_t)tok * a.ldx + base * 128 + v * 8);
+      if (a.pro == PRO_NORM) prw[j] = *reinterpret_cast<const uint4*>(a.norm_w + base * 128 + v * 8);
     }
   }
   if (a.pro == PRO_NORM) {

@@ -1,5 +1,6 @@
-"""Warp-wide instructions of the kernels, checked on their sources: undefined behaviour of this kind (a full-mask vote or an
-``.aligned`` instruction that some lanes of a warp do not execute) cannot be provoked safely on a GPU."""
+"""Rules of the kernels that are checked on their sources, since what breaks them (a full-mask vote or an ``.aligned``
+instruction that some lanes of a warp do not execute, a read that races with the kernel before) cannot be provoked safely
+or surely on a GPU."""
 import re
 from pathlib import Path
 
@@ -63,3 +64,13 @@ def test_loops_over_tensor_memory_bring_the_warp_together(path):
     bad = [line for body, line in _loops(s)
            if any(re.search(r"\b%s\s*\(" % r, body) for r in readers) and re.search(r"\bif\b", body) and "__syncwarp" not in body]
     assert not bad, bad
+
+
+@pytest.mark.parametrize("path", [p for p in SOURCES if p.name.startswith("wq_") and "pdl_wait()" in p.read_text()], ids=lambda p: p.name)
+def test_only_packed_weights_are_read_before_the_dependency_wait(path):
+    """Everything else a launch reads (activations, norm weights, statistics, residuals) may come from the kernel before."""
+    s = _code(path)
+    for m in re.finditer(r"__global__[^;{]*\{", s):
+        body = s[m.end() - 1:_close(s, m.end() - 1, "{}")]
+        before = body[:body.find("pdl_wait()")] if "pdl_wait()" in body else ""
+        assert not re.search(r"\b(a\.)?(norm_w|ss_in|resid|scratch|x)\s*(\[|\+\s*[a-z(])", before)
