@@ -78,3 +78,34 @@ def test_long_context_and_determinism():
     assert torch.equal(a, b)
     ref = _ref(q.float(), k.float(), v.float(), pos0, hq, hkv)
     assert (a.float().cpu().reshape(T, hq, 128) - ref).abs().max().item() < 0.03
+
+
+@pytest.mark.parametrize("hq,hkv,T,pos0", [(16, 2, 256, 3840), (8, 4, 300, 2000)])
+def test_probabilities_round_against_the_running_maximum(hq, hkv, T, pos0):
+    """The kernel is no further from fp64 than its scheme has to be: bf16 probabilities taken against the row's maximum so
+    far (a row's heaviest ones then lie at the top of a binade, where bf16 rounds best), everything else wider, the result
+    rounded to bf16.  Half a million outputs put the statistical error of a ratio below 0.2 %; a reference that lags behind
+    the maximum costs 2 %."""
+    torch.manual_seed(pos0)
+    n = pos0 + T
+    npg = (n + 15) // 16
+    k, v = torch.randn(npg * 16, hkv, 128, device=DEV).to(torch.bfloat16), torch.randn(npg * 16, hkv, 128, device=DEV).to(torch.bfloat16)
+    q = torch.randn(T, hq, 128, device=DEV).to(torch.bfloat16)
+    pool = torch.stack([x.view(npg, 16, hkv, 128).transpose(1, 2) for x in (k, v)], 1).contiguous()
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    out = A.attn_prefill_tc(q.reshape(T, -1), pool, torch.arange(npg, dtype=torch.int32, device=DEV)[None], 0, pos0, hq, hkv, status=status)
+    assert int(status.item()) == 0
+    kd, vd = k[:n].double().repeat_interleave(hq // hkv, 1), v[:n].double().repeat_interleave(hq // hkv, 1)
+    s = torch.einsum("thd,lhd->htl", q.double(), kd) / 128 ** 0.5
+    s = s.masked_fill(torch.arange(n, device=DEV) > (pos0 + torch.arange(T, device=DEV))[:, None], float("-inf"))
+    ref = torch.einsum("htl,lhd->thd", torch.softmax(s, -1), vd)
+    m = torch.full((hq, T, 1), float("-inf"), dtype=torch.float64, device=DEV)
+    o, l = torch.zeros(hq, T, 128, dtype=torch.float64, device=DEV), torch.zeros_like(m)
+    for b in range(0, n, 128):
+        sb = s[..., b:b + 128]
+        m2 = torch.maximum(m, sb.amax(-1, keepdim=True))
+        p, corr = torch.exp(sb - m2), torch.exp(m - m2)
+        o = o * corr + torch.einsum("htl,lhd->htd", p.to(torch.bfloat16).double(), vd[b:b + 128])
+        l, m = l * corr + p.sum(-1, keepdim=True), m2
+    scheme = (o / l).transpose(0, 1).to(torch.bfloat16).double()
+    assert (out.view(T, hq, 128).double() - ref).norm() < 1.006 * (scheme - ref).norm()
