@@ -80,7 +80,7 @@ def test_long_context_and_determinism():
     assert (a.float().cpu().reshape(T, hq, 128) - ref).abs().max().item() < 0.03
 
 
-@pytest.mark.parametrize("hq,hkv,T,pos0", [(16, 2, 256, 3840), (8, 4, 300, 2000)])
+@pytest.mark.parametrize("hq,hkv,T,pos0", [(16, 2, 256, 3840), (8, 4, 300, 2000), (64, 8, 330, 1000)])
 def test_probabilities_round_against_the_running_maximum(hq, hkv, T, pos0):
     """The kernel is no further from fp64 than its scheme has to be: bf16 probabilities taken against the row's maximum so
     far (a row's heaviest ones then lie at the top of a binade, where bf16 rounds best), everything else wider, the result

@@ -70,10 +70,10 @@ def test_gemv_work_split(n, k, bits, group):
     assert int(ws.status.item()) == 0 and int(ws.counters.abs().sum().item()) == 0
 
 
-# 128-row tiles, two per CTA, blocks of 128 keys: chunks that leave the second tile empty or ragged, contexts at and around
+# 128-row tiles, two per CTA (one up to 148 CTAs), blocks of 128 keys: chunks that leave the second tile empty or ragged, contexts at and around
 # a block's end, one to 128 query heads per KV head, scores that keep growing (the reference maximum moves several times)
 @pytest.mark.parametrize("T,pos0,hq,hkv,grow", [(1, 0, 8, 8, 0), (64, 63, 16, 8, 0), (64, 64, 16, 8, 0), (65, 64, 64, 8, 0), (300, 511, 8, 1, 0),
-                                                (130, 700, 16, 8, 1), (3, 250, 128, 1, 1)])
+                                                (130, 700, 16, 8, 1), (3, 250, 128, 1, 1), (330, 511, 64, 8, 0), (321, 64, 64, 8, 1)])
 def test_prefill_attention_tiles(T, pos0, hq, hkv, grow):
     """Against fp64; P is bf16 (relative 2^-9 per term, random), the result is rounded to bf16: below 6e-3 of the norm.
     Slots of the pool that the sequence does not use hold NaN."""
