@@ -78,6 +78,7 @@ constexpr int kCacheBytes = 160 * 1024;
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();                      // single lanes store just before; the barrier is .aligned
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {      // the same variable in CTA `rank`

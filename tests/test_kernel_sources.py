@@ -46,6 +46,14 @@ def test_no_warp_wide_instruction_under_a_lanes_own_wait(path):
     assert not bad, bad
 
 
+@pytest.mark.parametrize("path", [p for p in SOURCES if "barrier.cluster" in p.read_text()], ids=lambda p: p.name)
+def test_cluster_barriers_are_reached_by_whole_warps(path):
+    """barrier.cluster...aligned is executed by helpers that bring the warp together first."""
+    s = _code(path)
+    for m in re.finditer(r"barrier\.cluster\.arrive[\w.]*\.aligned", s):
+        assert "__syncwarp" in s[s.rindex("__device__", 0, m.start()):m.start()]
+
+
 def _loops(s):
     """(body, line) of every for loop."""
     for m in re.finditer(r"\bfor\s*\(", s):
