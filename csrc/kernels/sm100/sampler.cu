@@ -7,7 +7,8 @@
 // so "a draft is accepted iff it equals the target's own sample" gives the plain sampling distribution and, with a
 // seed, the same tokens with or without speculation and at any batch size.
 //
-// Implementation: a cluster of eight CTAs per row, each with an eighth of the row in shared memory.  Keys are the
+// Implementation: a cluster of CTAs per row (eight, fewer where many rows fill the chip anyway), each with its share of
+// the row in shared memory.  Keys are the
 // order-preserving integer images of the logits; top-k, top-p and the final inverse-CDF walk are radix descents over
 // 8-bit digits (4 passes each) with 256-bin histograms of counts or probability mass, summed over the cluster through
 // distributed shared memory; ties are broken by ascending token index.  Every sum is over integers, so the result does
@@ -72,12 +73,15 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-constexpr int kCl = 8;                 // CTAs per row
+constexpr int kMaxCl = 8;              // most CTAs per row
+constexpr int kSmsS = 148;
 constexpr int kListCap = 2048;         // survivors of the filters that a CTA keeps apart
 constexpr int kCacheBytes = 160 * 1024;
 
 __device__ __forceinline__ uint32_t cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+template <int CL>
 __device__ __forceinline__ void cluster_sync() {
+  if (CL == 1) { __syncthreads(); return; }
   __syncwarp();                      // single lanes store just before; the barrier is .aligned
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -132,14 +136,14 @@ __device__ __forceinline__ void scan_share(const Share& s, F f) {
   }
 }
 
-enum ClOp { CL_SUM, CL_MAXF, CL_MIN };
+enum ClOp { CL_SUM, CL_MAX, CL_MIN };
 // Reduction of one 64-bit value per thread over the CTA and the cluster; every thread gets the result.
-template <ClOp OP>
+template <ClOp OP, int CL>
 __device__ unsigned long long cluster_reduce(Share& s, unsigned long long v) {
   auto comb = [](unsigned long long a, unsigned long long b) -> unsigned long long {
     if (OP == CL_SUM) return a + b;
     if (OP == CL_MIN) return a < b ? a : b;
-    return (unsigned long long)__float_as_uint(fmaxf(__uint_as_float((uint32_t)a), __uint_as_float((uint32_t)b)));
+    return a > b ? a : b;
   };
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = comb(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -153,17 +157,17 @@ __device__ unsigned long long cluster_reduce(Share& s, unsigned long long v) {
     for (int o = 16; o > 0; o >>= 1) v = comb(v, __shfl_xor_sync(0xffffffffu, v, o));
     if (threadIdx.x == 0) s.xch[t] = v;
   }
-  cluster_sync();
+  cluster_sync<CL>();
   v = peer_u64(peer_addr(&s.xch[t], 0));
 #pragma unroll
-  for (uint32_t r = 1; r < kCl; ++r) v = comb(v, peer_u64(peer_addr(&s.xch[t], r)));
+  for (uint32_t r = 1; r < CL; ++r) v = comb(v, peer_u64(peer_addr(&s.xch[t], r)));
   return v;
 }
 
 // Radix descent: finds the largest key prefix such that the mass of all elements with a strictly larger key is
 // <= target (mass = probability or count).  On return *above = mass strictly above the final key.
 // `keep_min`: elements with key < keep_min are ignored.
-template <bool COUNT>
+template <bool COUNT, int CL>
 __device__ uint32_t radix_descend(Share& s, float mx, float inv_t, uint32_t keep_min, unsigned long long target,
                                   unsigned long long* above_out) {
   uint32_t prefix = 0, mask = 0;
@@ -196,14 +200,14 @@ __device__ uint32_t radix_descend(Share& s, float mx, float inv_t, uint32_t keep
       }
       if (on && !big) hist_add(hist, dig, v);
     });
-    cluster_sync();
+    cluster_sync<CL>();
     // the row's digit d, walked from high to low, is the first with above + mass(digits >= d) > target (0 if none):
     // thread i < 256 takes digit 255 - i, so the running masses are prefix sums over the threads
     unsigned long long h = 0, inc = 0;
     if (threadIdx.x < 256) {
       const int d = 255 - (int)threadIdx.x;
 #pragma unroll
-      for (uint32_t r = 0; r < kCl; ++r) {
+      for (uint32_t r = 0; r < CL; ++r) {
         const uint32_t lo = peer_u32(peer_addr(&hist.lo[d], r)), hi = peer_u32(peer_addr(&hist.hi[d], r));
         h += ((unsigned long long)hi << 32) | lo;
       }
@@ -235,6 +239,44 @@ __device__ uint32_t radix_descend(Share& s, float mx, float inv_t, uint32_t keep
   return prefix;
 }
 
+// The maximum of a row and its lowest index; NaNs are passed over.
+struct Best {
+  float v = -INFINITY;
+  int i = 0x7fffffff;
+  __device__ __forceinline__ void see(float x, int at) {
+    if (x > v || (x == v && at < i)) { v = x; i = at; }
+  }
+  // As one integer that grows with the value and falls with the index (-0 counts as +0).
+  __device__ __forceinline__ unsigned long long packed() const { return ((unsigned long long)key_of(v + 0.f) << 32) | (0xffffffffu - (uint32_t)i); }
+};
+__device__ __forceinline__ float packed_value(unsigned long long p) {
+  const uint32_t k = (uint32_t)(p >> 32);
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+__device__ __forceinline__ int packed_index(unsigned long long p) { return (int)(0xffffffffu - (uint32_t)p); }
+
+// Elements x[0 .. n) of a row (index lo on) as this thread sees them, four at a time where the alignment allows it; kept
+// in `cache` if that is given.
+__device__ __forceinline__ void load_share(const float* x, int n, int lo, float* cache, Best& b) {
+  int i0 = 0;
+  if ((reinterpret_cast<uintptr_t>(x) & 15) == 0) {
+    const int n4 = n >> 2;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n4; i += kThreads) {
+      const float4 v = reinterpret_cast<const float4*>(x)[i];
+      if (cache) reinterpret_cast<float4*>(cache)[i] = v;
+      const int at = lo + 4 * i;
+      b.see(v.x, at); b.see(v.y, at + 1); b.see(v.z, at + 2); b.see(v.w, at + 3);
+    }
+    i0 = 4 * n4;
+  }
+  for (int i = i0 + threadIdx.x; i < n; i += kThreads) {
+    const float v = x[i];
+    if (cache) cache[i] = v;
+    b.see(v, lo + i);
+  }
+}
+
 }  // namespace
 
 // Determinism: counts and fixed-point masses are integers, so every histogram, threshold and the final walk are
@@ -243,8 +285,10 @@ __device__ uint32_t radix_descend(Share& s, float mx, float inv_t, uint32_t keep
 // What bounds it: about fifteen passes over the row.  With one CTA per row (the earlier kernel) a pass moved 600 KB of
 // logits from L2 through a single SM and walked its 256 bins serially on every thread: 518 us for 16 rows of 151936
 // logits.  Here a row is read from memory once, a pass costs 19 values per thread plus a cluster barrier, and passes
-// after top-k or min-p touch the survivors only: 93 us.
-__global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_rows_kernel(const SampleArgs a, int share, int cached) {
+// after top-k or min-p touch the survivors only: 92 us.  A greedy row is the load and one exchange (1 row 6.9 -> 4.3 us).
+// CACHED: the share is in shared memory (known at compile time, so that the passes use shared-memory loads).
+template <int CL, bool CACHED>
+__global__ void __launch_bounds__(kThreads) sample_rows_kernel(const SampleArgs a, int share, int solo) {
   extern __shared__ __align__(16) float cache[];
   __shared__ Hist hist[2];
   __shared__ unsigned long long xch[2], warp64[kThreads / 32], pickv[2];
@@ -253,8 +297,8 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
   __shared__ int s_pick, s_list;
   pdl_wait();
   pdl_launch_dependents();
-  const int row = blockIdx.x / kCl;
-  const int rank = (int)cluster_rank();
+  const int row = blockIdx.x / CL;
+  const int rank = CL == 1 ? 0 : (int)cluster_rank();
   Share s;
   s.lo = min(rank * share, a.vocab);
   s.n = min(share, a.vocab - s.lo);
@@ -262,37 +306,26 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
   s.hist = hist; s.xch = xch; s.warp64 = warp64; s.pick = &s_pick; s.pickv = pickv;
   s.turn = 0;
   const float* gx = a.logits + (size_t)row * a.ld + s.lo;
-  s.x = gx;
-  float mx = -INFINITY;
-  if (cached) {
-    int i0 = 0;
-    if ((reinterpret_cast<uintptr_t>(gx) & 15) == 0) {
-      const int n4 = s.n >> 2;
-#pragma unroll 4
-      for (int i = threadIdx.x; i < n4; i += kThreads) {
-        const float4 v = reinterpret_cast<const float4*>(gx)[i];
-        reinterpret_cast<float4*>(cache)[i] = v;
-        mx = fmaxf(fmaxf(mx, fmaxf(v.x, v.y)), fmaxf(v.z, v.w));
-      }
-      i0 = 4 * n4;
-    }
-    for (int i = i0 + threadIdx.x; i < s.n; i += kThreads) { const float v = gx[i]; cache[i] = v; mx = fmaxf(mx, v); }
-    s.x = cache;
-  } else {
-    for (int i = threadIdx.x; i < s.n; i += kThreads) mx = fmaxf(mx, gx[i]);
-  }
-  mx = __uint_as_float((uint32_t)cluster_reduce<CL_MAXF>(s, __float_as_uint(mx)));     // its barriers also publish `cache` to the CTA
+  if (CACHED) s.x = cache;
+  else s.x = gx;
   const float T = a.temperature ? a.temperature[row] : 0.f;
   const int topk = a.top_k ? a.top_k[row] : 0;
-  auto lowest_max = [&]() {          // lowest index among the maxima
-    unsigned long long best = 0x7fffffffull;
-    scan_share(s, [&](float xv, int i, bool valid) { if (valid && xv == mx) best = min(best, (unsigned long long)i); });
-    best = cluster_reduce<CL_MIN>(s, best);
-    if (rank == 0 && threadIdx.x == 0) a.out[row] = (int)best;
-  };
-  if (T <= 0.f || topk == 1) {       // greedy
-    lowest_max();
-    cluster_sync();                  // no CTA leaves while another still reads its shared memory
+  const bool greedy = T <= 0.f || topk == 1;
+  Best best;
+  if (solo && greedy) {              // the first CTA alone; the others make room
+    if (rank == 0) {
+      load_share(gx, a.vocab, 0, nullptr, best);
+      const unsigned long long top = cluster_reduce<CL_MAX, 1>(s, best.packed());
+      if (threadIdx.x == 0) a.out[row] = packed_index(top);
+    }
+    return;
+  }
+  load_share(gx, s.n, s.lo, CACHED ? cache : nullptr, best);
+  const unsigned long long top = cluster_reduce<CL_MAX, CL>(s, best.packed());         // its barriers also publish `cache` to the CTA
+  const float mx = packed_value(top);
+  if (greedy) {
+    if (rank == 0 && threadIdx.x == 0) a.out[row] = packed_index(top);
+    cluster_sync<CL>();              // no CTA leaves while another still reads its shared memory
     return;
   }
   const float inv_t = 1.f / T;
@@ -303,7 +336,7 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
   // top-k: key of the k-th largest logit (ties at the threshold are all kept; the index rule orders them)
   if (topk > 1 && topk < a.vocab) {
     unsigned long long above;
-    const uint32_t kth = radix_descend<true>(s, mx, inv_t, 0u, (unsigned long long)(topk - 1), &above);
+    const uint32_t kth = radix_descend<true, CL>(s, mx, inv_t, 0u, (unsigned long long)(topk - 1), &above);
     keep_min = max(keep_min, kth);
   }
   if (keep_min > 0) {                // later passes read this CTA's survivors only, if there is room for them
@@ -321,14 +354,14 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
   auto mass_left = [&]() {           // mass of what is left
     unsigned long long z = 0;
     scan_share(s, [&](float xv, int, bool valid) { if (valid && key_of(xv) >= keep_min) z += mass_of(xv, mx, inv_t); });
-    return cluster_reduce<CL_SUM>(s, z);
+    return cluster_reduce<CL_SUM, CL>(s, z);
   };
   // top-p over what is left: smallest descending prefix whose mass reaches top_p * Z
   const float topp = a.top_p ? a.top_p[row] : 1.f;
   if (topp < 1.f) {
     const unsigned long long z = mass_left();
     unsigned long long above;
-    const uint32_t cut = radix_descend<false>(s, mx, inv_t, keep_min, (unsigned long long)((double)topp * (double)z), &above);
+    const uint32_t cut = radix_descend<false, CL>(s, mx, inv_t, keep_min, (unsigned long long)((double)topp * (double)z), &above);
     keep_min = max(keep_min, cut);
   }
   // draw
@@ -338,17 +371,16 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
   unsigned long long target = (unsigned long long)(u * (double)z);
   if (z > 0 && target >= z) target = z - 1;
   unsigned long long above;
-  const uint32_t key = radix_descend<false>(s, mx, inv_t, keep_min, target, &above);
+  const uint32_t key = radix_descend<false, CL>(s, mx, inv_t, keep_min, target, &above);
   // among the tokens that share the final key, walk by ascending index: the `want`-th of them wins
   const unsigned long long w = mass_of(__uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key), mx, inv_t);
   const unsigned long long rank64 = w > 0 && target > above ? (target - above) / w : 0ull;
   const int nth = (int)(rank64 > 1000000000ull ? 1000000000ull : rank64);
   unsigned long long same = 0;
   scan_share(s, [&](float xv, int, bool valid) { same += valid && key_of(xv) == key ? 1u : 0u; });
-  const int cnt = (int)cluster_reduce<CL_SUM>(s, same);
+  const int cnt = (int)cluster_reduce<CL_SUM, CL>(s, same);
   if (cnt == 0) {                                            // rounding pushed the walk past the last bin: take the mode
-    s.ln = -1;
-    lowest_max();
+    if (rank == 0 && threadIdx.x == 0) a.out[row] = packed_index(top);
   } else if (cnt == 1) {                                     // the usual case: one token owns the key
     scan_share(s, [&](float xv, int i, bool valid) { if (valid && key_of(xv) == key) a.out[row] = i; });
   } else {
@@ -359,12 +391,12 @@ __global__ void __cluster_dims__(kCl, 1, 1) __launch_bounds__(kThreads) sample_r
       const int mid = (lo + hi) >> 1;
       unsigned long long c = 0;
       scan_share(s, [&](float xv, int i, bool valid) { c += valid && i <= mid && key_of(xv) == key ? 1u : 0u; });
-      c = cluster_reduce<CL_SUM>(s, c);
+      c = cluster_reduce<CL_SUM, CL>(s, c);
       if ((int)c >= want + 1) hi = mid; else lo = mid + 1;
     }
     if (rank == 0 && threadIdx.x == 0) a.out[row] = lo;
   }
-  cluster_sync();
+  cluster_sync<CL>();                // no CTA leaves while another still reads its shared memory
 }
 
 // Longest-prefix acceptance for one or more verify blocks.  Block b covers rows [row0[b], row0[b] + cnt[b]): row 0 is
@@ -387,19 +419,39 @@ __global__ void spec_accept_kernel(const int* __restrict__ ids, const int* __res
 
 using namespace b2;
 
-B2_API int b2_sample_rows(const SampleArgs* a, int rows, cudaStream_t st) {
-  if (!a || rows <= 0 || a->vocab <= 0 || !a->logits || !a->out) return B2_ERR_ARG;
-  const int share = ((a->vocab + kCl - 1) / kCl + 3) & ~3;             // multiple of four: shares keep the row's alignment
-  const int cached = (long)share * 4 <= kCacheBytes;
-  if (cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCacheBytes) != cudaSuccess) return B2_ERR_LAUNCH;
+template <int CL, bool CACHED>
+static int sample_launch(const SampleArgs& a, int rows, int share, int solo, cudaStream_t st) {
+  auto kern = sample_rows_kernel<CL, CACHED>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCacheBytes) != cudaSuccess) return B2_ERR_LAUNCH;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)rows * kCl); cfg.blockDim = dim3(kThreads); cfg.stream = st;
-  cfg.dynamicSmemBytes = cached ? (size_t)share * 4 : 0;
-  cudaLaunchAttribute at[1];
+  cfg.gridDim = dim3((unsigned)rows * CL); cfg.blockDim = dim3(kThreads); cfg.stream = st;
+  cfg.dynamicSmemBytes = CACHED ? (size_t)share * 4 : 0;
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, sample_rows_kernel, *a, share, cached) == cudaSuccess ? B2_OK : B2_ERR_LAUNCH;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = CL; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = CL == 1 ? 1 : 2;
+  return cudaLaunchKernelEx(&cfg, kern, a, share, solo) == cudaSuccess ? B2_OK : B2_ERR_LAUNCH;
+}
+
+B2_API int b2_sample_rows(const SampleArgs* a, int rows, cudaStream_t st) {
+  if (!a || rows <= 0 || a->vocab <= 0 || !a->logits || !a->out) return B2_ERR_ARG;
+  // CTAs per row: eight, or fewer where a share would have fewer values than threads (1000 logits, greedy: 4.4 -> 2.7 us),
+  // or where eight would not all be resident at once (two per SM, by their shared memory) and fewer still are.  Where they
+  // come in waves all the same, a greedy row, which is one short pass, is left to one CTA.  128 rows, always eight -> by
+  // this rule: greedy 151936 logits 44 -> 21 us (one CTA per row 13), 32000 28 -> 6 (5); top-p 32000 193 -> 96 (164).
+  auto share_of = [&](int c) { return ((a->vocab + c - 1) / c + 3) & ~3; };   // multiple of four: shares keep the row's alignment
+  auto two = [&](int c) { return (long)share_of(c) * 4 <= 88 * 1024; };
+  auto waves = [&](int c) { return (long)rows * c > (two(c) ? 2L : 1L) * kSmsS; };
+  int cl = kMaxCl;
+  while (cl > 1 && (share_of(cl) < kThreads || (waves(cl) && two(cl / 2)))) cl /= 2;
+  const int solo = waves(cl);
+  const int share = share_of(cl);
+  if (cl == 4) return sample_launch<4, true>(*a, rows, share, solo, st);
+  if (cl == 2) return sample_launch<2, true>(*a, rows, share, solo, st);
+  if (cl == 1) return sample_launch<1, true>(*a, rows, share, solo, st);
+  return (long)share * 4 <= kCacheBytes ? sample_launch<8, true>(*a, rows, share, solo, st) : sample_launch<8, false>(*a, rows, share, solo, st);
 }
 
 B2_API int b2_spec_accept(const int* ids, const int* target, const int* row0, const int* cnt, int n_blocks, int* n_emitted,

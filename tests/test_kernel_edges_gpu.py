@@ -134,3 +134,26 @@ def test_gemm_tiles(M, N, K):
     ref = a.double() @ b.double().t()
     assert int(status.item()) == 0
     assert (d.double() - ref).norm() < 1e-5 * ref.norm()
+
+
+# CTAs per row: eight (with greedy rows on one), four, two and one, by rows and vocabulary, more of them for a row on its own
+@pytest.mark.parametrize("rows,vocab,ld", [(40, 190001, 190004), (80, 20000, 20000), (50, 40000, 40000), (80, 20001, 20003), (300, 1000, 1000), (300, 7, 9)])
+def test_sampler_rows_do_not_depend_on_their_company(rows, vocab, ld):
+    torch.manual_seed(rows)
+    buf = torch.zeros(rows, ld, device=DEV)
+    x = torch.randn(rows, vocab, device=DEV) * 3
+    x[1::3] = torch.round(x[1::3])
+    x[2::5, ::2] = float("-inf")
+    x[4] = float("-inf")
+    x[9, : vocab // 2] = float("nan")
+    buf[:, :vocab] = x
+    i = list(range(rows))
+    T, k, p, mp = [0.0 if j % 4 == 0 or j == 9 else 0.6 + 0.1 * (j % 5) for j in i], [(0, 1, 40, 3)[j % 4] for j in i], [(1.0, 0.9, 0.5)[j % 3] for j in i], [(0.0, 0.05)[j % 2] for j in i]
+    seeds, pos = [99 + j for j in i], [7 * j for j in i]
+    args = _params(DEV, rows, T, k, p, mp, seeds, pos)
+    out = basic.sample_rows(buf, *args, n_valid=vocab).cpu()
+    one = [int(basic.sample_rows(buf[j:j + 1], *(a[j:j + 1].contiguous() for a in args), n_valid=vocab)) for j in i]
+    assert out.tolist() == one
+    greedy = [j for j in i if T[j] == 0.0 and j != 9]
+    assert out[greedy].tolist() == x[greedy].argmax(-1).tolist()
+    assert int(out[9]) == vocab // 2 + int(x[9, vocab // 2:].argmax())
