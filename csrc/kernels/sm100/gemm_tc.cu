@@ -143,6 +143,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int nkb = (g.K + BK - 1) / BK;
 
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     for (int i = 0; i < kStagesG; ++i) { mbar_init_g(smem_u32(&full_bar[i]), 1); mbar_init_g(smem_u32(&empty_bar[i]), 1); }
     for (int i = 0; i < 2; ++i) { mbar_init_g(smem_u32(&acc_full[i]), 1); mbar_init_g(smem_u32(&acc_empty[i]), 4); }
     s_failed = 0;
