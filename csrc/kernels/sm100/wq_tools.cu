@@ -73,64 +73,60 @@ __device__ __forceinline__ unsigned fm_load_code(const uint8_t* wq, const FmPos&
   return c;
 }
 
-// FM -> bf16.  One warp per (32-row panel, 128-k batch) block: a lane reads its fragments (16-byte loads, the block is
-// contiguous), one lop3 and one exact fp16 FMA give two codes, and w = (code - zero) * scale is formed in fp32 and
-// rounded once.  A store of the warp covers eight rows x 32 bytes, whole DRAM sectors.  Bound by the bf16 writes (two
-// bytes a weight against 0.27 to 0.53 read); the earlier kernel, one thread per four codes, spent its time on the
-// index arithmetic of every code (gate_up 51200 x 5120, 4 bits: 530 us there, 120 us here; floor 101 us).
+// FM -> bf16.  One warp per 16-row half of a (32-row panel, 128-k batch) block: a lane reads its fragments (16-byte loads,
+// a half is two contiguous pieces), one lop3 and one exact fp16 FMA give two codes, and w = (code - zero) * scale is formed
+// in fp32 and rounded once.  A store of the warp covers eight rows x 32 bytes, whole DRAM sectors.  Bound by the bf16 writes
+// (two bytes a weight against 0.27 to 0.53 read); the earlier kernel, one thread per four codes, spent its time on the index
+// arithmetic of every code.  4 bits, group 128, that kernel -> one warp per block -> this: 51200 x 5120 526 -> 114 -> 107 us
+// (floor 101), 1024 x 1024 4.6 -> 3.4 -> 2.5, 256 x 512 2.2 -> 3.2 -> 2.4 (a warp's code is straight-line and runs once).
 // A16: the packed buffer is 16-byte aligned (every linear that the engine loads); otherwise the words come one by one.
 template <int BITS, int GROUP, bool A16>
 __global__ void __launch_bounds__(256) wq_dequant_kernel(const uint8_t* __restrict__ wq, int npan, int nbat, bf16* __restrict__ out, long ldo) {
   constexpr int GPB = 128 / GROUP;
   using R = Ring<BITS, GROUP, 2>;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const long blk = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (blk >= (long)npan * nbat) return;
-  const int pan = (int)(blk / nbat), batch = (int)(blk - (long)pan * nbat);
+  const unsigned blk = blockIdx.x * 4 + (threadIdx.x >> 6);
+  if (blk >= (unsigned)npan * (unsigned)nbat) return;
+  const unsigned pan = blk / (unsigned)nbat, batch = blk - pan * (unsigned)nbat;
+  const int r = (threadIdx.x >> 5) & 1;
   const uint8_t* src = wq + (size_t)blk * R::BLK;
-  WFrag<BITS, GROUP> cf[2];
+  WFrag<BITS, GROUP> cf;
+  const uint8_t* wrec = src + r * R::W_BATCH;
+  const uint8_t* szrec = src + 2 * R::W_BATCH + r * GPB * 64;
+  if (A16) {
+    load_frag_smem<BITS, GROUP>(cf, wrec, szrec, lane);
+  } else {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(wrec);
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const uint8_t* wrec = src + r * R::W_BATCH;
-    const uint8_t* szrec = src + 2 * R::W_BATCH + r * GPB * 64;
-    if (A16) {
-      load_frag_smem<BITS, GROUP>(cf[r], wrec, szrec, lane);
-    } else {
-      const uint32_t* w = reinterpret_cast<const uint32_t*>(wrec);
-#pragma unroll
-      for (int i = 0; i < R::RPB; ++i) {
-        const uint32_t* q = w + i * (Fmt<BITS>::REC / 4) + lane * 4;
-        cf[r].lo[i] = make_uint4(q[0], q[1], q[2], q[3]);
-      }
-      if (BITS == 3) cf[r].hi = make_uint2(w[128 + lane * 2], w[128 + lane * 2 + 1]);
-      const uint32_t* z = reinterpret_cast<const uint32_t*>(szrec);
-#pragma unroll
-      for (int i = 0; i < GPB; ++i) { cf[r].sz[i][0] = z[i * 16 + g]; cf[r].sz[i][1] = z[i * 16 + 8 + g]; }
+    for (int i = 0; i < R::RPB; ++i) {
+      const uint32_t* q = w + i * (Fmt<BITS>::REC / 4) + lane * 4;
+      cf.lo[i] = make_uint4(q[0], q[1], q[2], q[3]);
     }
+    if (BITS == 3) cf.hi = make_uint2(w[128 + lane * 2], w[128 + lane * 2 + 1]);
+    const uint32_t* z = reinterpret_cast<const uint32_t*>(szrec);
+#pragma unroll
+    for (int i = 0; i < GPB; ++i) { cf.sz[i][0] = z[i * 16 + g]; cf.sz[i][1] = z[i * 16 + 8 + g]; }
   }
+  bf16* o = out + (size_t)(pan * 32 + r * 16 + g) * ldo + (size_t)batch * 128 + 4 * t;
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    bf16* o = out + (size_t)(pan * 32 + r * 16 + g) * ldo + (size_t)batch * 128 + 4 * t;
+  for (int s = 0; s < 8; ++s) {
+    const int gi = s * GPB / 8;
+    uint32_t af[4];
+    extract<BITS, GROUP>(cf, s, af);
+    // 1024 + c * code -> code: exact in fp16 (c = 1, 4, 16, 64)
+    const float c0 = BITS == 4 ? 1.f : ((s & 1) ? 1.f / 16.f : 1.f), c1 = BITS == 4 ? 1.f / 16.f : ((s & 1) ? 1.f / 64.f : 1.f / 4.f);
 #pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const int gi = s * GPB / 8;
-      uint32_t af[4];
-      extract<BITS, GROUP>(cf[r], s, af);
-      // 1024 + c * code -> code: exact in fp16 (c = 1, 4, 16, 64)
-      const float c0 = BITS == 4 ? 1.f : ((s & 1) ? 1.f / 16.f : 1.f), c1 = BITS == 4 ? 1.f / 16.f : ((s & 1) ? 1.f / 64.f : 1.f / 4.f);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {            // rows g and g + 8
-        const float2 sz = __half22float2(*reinterpret_cast<const __half2*>(&cf[r].sz[gi][h]));
-        const __half2 v0 = __hfma2(*reinterpret_cast<const __half2*>(&af[h]), __float2half2_rn(c0), __float2half2_rn(-1024.f * c0));
-        const __half2 v1 = __hfma2(*reinterpret_cast<const __half2*>(&af[2 + h]), __float2half2_rn(c1), __float2half2_rn(-1024.f * c1));
-        const float2 f0 = __half22float2(v0), f1 = __half22float2(v1);
-        const __nv_bfloat162 p0 = __floats2bfloat162_rn((f0.x - sz.y) * sz.x, (f0.y - sz.y) * sz.x);
-        const __nv_bfloat162 p1 = __floats2bfloat162_rn((f1.x - sz.y) * sz.x, (f1.y - sz.y) * sz.x);
-        uint2 w;
-        w.x = *reinterpret_cast<const uint32_t*>(&p0);
-        w.y = *reinterpret_cast<const uint32_t*>(&p1);
-        *reinterpret_cast<uint2*>(o + (size_t)h * 8 * ldo + s * 16) = w;
-      }
+    for (int h = 0; h < 2; ++h) {            // rows g and g + 8
+      const float2 sz = __half22float2(*reinterpret_cast<const __half2*>(&cf.sz[gi][h]));
+      const __half2 v0 = __hfma2(*reinterpret_cast<const __half2*>(&af[h]), __float2half2_rn(c0), __float2half2_rn(-1024.f * c0));
+      const __half2 v1 = __hfma2(*reinterpret_cast<const __half2*>(&af[2 + h]), __float2half2_rn(c1), __float2half2_rn(-1024.f * c1));
+      const float2 f0 = __half22float2(v0), f1 = __half22float2(v1);
+      const __nv_bfloat162 p0 = __floats2bfloat162_rn((f0.x - sz.y) * sz.x, (f0.y - sz.y) * sz.x);
+      const __nv_bfloat162 p1 = __floats2bfloat162_rn((f1.x - sz.y) * sz.x, (f1.y - sz.y) * sz.x);
+      uint2 w;
+      w.x = *reinterpret_cast<const uint32_t*>(&p0);
+      w.y = *reinterpret_cast<const uint32_t*>(&p1);
+      *reinterpret_cast<uint2*>(o + (size_t)h * 8 * ldo + s * 16) = w;
     }
   }
 }
@@ -285,7 +281,7 @@ B2_API int b2_wq_dequant(const uint8_t* wq, int n, int k, int bits, int group, b
     case 2128: kern = a16 ? wq_dequant_kernel<2, 128, true> : wq_dequant_kernel<2, 128, false>; break;
     default: kern = a16 ? wq_dequant_kernel<2, 64, true> : wq_dequant_kernel<2, 64, false>; break;
   }
-  kern<<<(unsigned)(((long)npan * nbat + 7) / 8), 256, 0, stream>>>(wq, npan, nbat, out, ldo);
+  kern<<<(unsigned)(((long)npan * nbat + 3) / 4), 256, 0, stream>>>(wq, npan, nbat, out, ldo);
   return cudaGetLastError() == cudaSuccess ? B2_OK : B2_ERR_LAUNCH;
 }
 
