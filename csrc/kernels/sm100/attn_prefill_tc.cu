@@ -131,11 +131,6 @@ __device__ __forceinline__ bool pf_wait_warp(uint32_t bar, uint32_t parity) {
   }
   return __all_sync(0xffffffffu, ok) != 0;
 }
-__device__ __forceinline__ bool pf_elect() {
-  uint32_t ok;
-  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok));
-  return ok != 0;
-}
 __device__ __forceinline__ void pf_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void pf_expect(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -275,7 +270,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tc_kernel(const __
     };
     bool ok = pf_wait_warp(smem_u32(&k_full[0]), 0);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && pf_elect()) {
+    if (ok && lane == 0) {
       issue_s(0, 0);
       if (TILES == 2) issue_s(1, 0);
       pf_commit(smem_u32(&k_empty[0]));
@@ -290,7 +285,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tc_kernel(const __
         if (t == 0 && j + 1 < nb) ok = ok && pf_wait_warp(smem_u32(&k_full[sn]), (uint32_t)((j + 1) >> 1) & 1u);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (pf_elect()) {
+        if (lane == 0) {
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             pf_mma_ts(tmem + 256u + (uint32_t)t * 128u, tmem + (uint32_t)t * 128u + (uint32_t)k * 8u,
