@@ -660,11 +660,9 @@ __device__ __forceinline__ void gemv_body(const StepArgs& a, const Phase& ph, ui
       int freed = usz;
       if (ring.cpos + usz > kRingBytes) { freed += kRingBytes - ring.cpos; ring.cpos = 0; }
       B2_T0(tw0);
-      if (!failed) {
-        if (!mbar_wait_bounded(ring.bars_u + (ring.cidx % kRingBars) * 8, (ring.cidx / kRingBars) & 1u)) {
-          atomicExch(a.status, (int)B2_ERR_TIMEOUT);
-          failed = true;
-        }
+      if (!failed && !mbar_wait_warp(ring.bars_u + (ring.cidx % kRingBars) * 8, (ring.cidx / kRingBars) & 1u)) {   // voted: the
+        if (lane == 0) atomicExch(a.status, (int)B2_ERR_TIMEOUT);                                                   // mma are .aligned
+        failed = true;
       }
       B2_TC(tc_wait, tw0);
       B2_T0(tc0);

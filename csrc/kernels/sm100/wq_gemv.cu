@@ -209,8 +209,8 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
 #pragma unroll 1
     for (int b = b_lo; b < b_hi; ++b) {
       const int slot = cons % NST;
-      if (!mbar_wait_bounded(bars_u + slot * 8, (cons / NST) & 1u)) {
-        if (a.status) atomicExch(a.status, (int)B2_ERR_TIMEOUT);
+      if (!mbar_wait_warp(bars_u + slot * 8, (cons / NST) & 1u)) {   // voted: the mma below are .aligned
+        if (a.status && lane == 0) atomicExch(a.status, (int)B2_ERR_TIMEOUT);
         failed = true;
         break;
       }

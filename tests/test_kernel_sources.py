@@ -46,6 +46,17 @@ def test_no_warp_wide_instruction_under_a_lanes_own_wait(path):
     assert not bad, bad
 
 
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_waits_of_whole_warps_are_voted(path):
+    """Lanes may leave a wait at different tries, so outside the wait helpers a wait is either voted or run by one lane:
+    the mma and tcgen05 instructions behind it are .aligned."""
+    s = _code(path)
+    alone = [(s.index(body), s.index(body) + len(body)) for cond, body, _ in _branches(s) if "lane == 0" in cond]
+    helpers = [(m.start(), _close(s, m.end() - 1, "{}")) for m in re.finditer(r"\bbool\s+\w*(mbar|pf)_\w+\([^)]*\)\s*\{", s)]
+    bad = [s.count("\n", 0, m.start()) + 1 for m in LANE_WAIT.finditer(s) if not any(a <= m.start() < b for a, b in alone + helpers)]
+    assert not bad, bad
+
+
 @pytest.mark.parametrize("path", [p for p in SOURCES if "barrier.cluster" in p.read_text()], ids=lambda p: p.name)
 def test_cluster_barriers_are_reached_by_whole_warps(path):
     """barrier.cluster...aligned is executed by helpers that bring the warp together first."""
