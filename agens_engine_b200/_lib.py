@@ -111,9 +111,7 @@ class WqGemvArgs(C.Structure):
         ("amax_val", C.c_void_p), ("amax_idx", C.c_void_p), ("n_valid", C.c_int),
         ("scratch", C.c_void_p), ("counters", C.c_void_p),
         ("status", C.c_void_p),
-        ("debug", C.c_int),
         ("tp", TpPush),
-        ("trace", C.c_void_p),
     ]
 
 

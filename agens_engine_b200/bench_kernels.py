@@ -85,36 +85,29 @@ def bench_gemv(args):
     dev = "cuda:0"
     pk = peaks()
     ws = L.GemvWorkspace(dev, floats=16 << 20)
-    ws.mm_min_rows = 33                      # times the GEMV family itself; above 8 rows its activation staging only fits small k slices
+    ws.mm_min_rows = 33                      # times the GEMV itself at every row count (eight rows at a time)
     shapes = [("qkv", 10240, 5120), ("o", 5120, 8192), ("gate_up", 51200, 5120), ("down", 5120, 25600),
               ("lm_head", 151936, 5120)]
     if args.small:
         shapes = [("gate_up", 51200, 5120)]
-    rows = []
     for name, n, k in shapes:
         for bits in ([4] if name == "lm_head" else [2, 3, 4]):
-            for _ in (0,):
-                ks_list = sorted({1, L.choose_ks(n, k), L.choose_ks(n, k, 1280), L.choose_ks(n, k, 5120)})
-                for ks in ks_list:
-                    lin = L.WqLinear.random(n, k, bits, 128, dev, seed=1, ks=ks)
-                    nbytes = lin.nbytes()
-                    ncopy = max(2, min(24, (512 << 20) // nbytes + 1))   # rotate over > 512 MiB of weights: L2 stays cold
-                    lins = [lin] + [L.WqLinear(n, k, bits, 128, lin.wq.clone(), ks, lin.rb)
-                                    for _ in range(ncopy - 1)]
-                    x = torch.randn(args.m, k, device=dev).to(torch.bfloat16)
-                    out = torch.empty(args.m, n, dtype=torch.bfloat16, device=dev)
+            lin = L.WqLinear.random(n, k, bits, 128, dev, seed=1)
+            nbytes = lin.nbytes()
+            ncopy = max(2, min(24, (512 << 20) // nbytes + 1))   # rotate over > 512 MiB of weights: L2 stays cold
+            lins = [lin] + [L.WqLinear(n, k, bits, 128, lin.wq.clone(), lin.ks, lin.rb) for _ in range(ncopy - 1)]
+            x = torch.randn(args.m, k, device=dev).to(torch.bfloat16)
+            out = torch.empty(args.m, n, dtype=torch.bfloat16, device=dev)
 
-                    def launch_all():
-                        for ln in lins:
-                            L.gemv(ln, x, ws, out=out)
+            def launch_all():
+                for ln in lins:
+                    L.gemv(ln, x, ws, out=out)
 
-                    med, best = graph_time_us(launch_all, len(lins))
-                    gbs = nbytes / med / 1e3
-                    rows.append(dict(name=name, n=n, k=k, bits=bits, ks=ks, m=args.m, us=round(med, 2),
-                                     best_us=round(best, 2), gbs=round(gbs, 1), frac=round(gbs / pk["hbm_gbs"], 3),
-                                     copies=ncopy))
-                    print(json.dumps(rows[-1]), flush=True)
-                    del lins
+            med, best = graph_time_us(launch_all, len(lins))
+            gbs = nbytes / med / 1e3
+            print(json.dumps(dict(name=name, n=n, k=k, bits=bits, m=args.m, us=round(med, 2), best_us=round(best, 2), gbs=round(gbs, 1),
+                                  frac=round(gbs / pk["hbm_gbs"], 3), copies=ncopy)), flush=True)
+            del lins
     print(json.dumps({"peaks": pk, "timing": "CUDA graph of back-to-back launches over rotating weight copies "
                       "(> 512 MiB, larger than L2); median per launch"}))
 
@@ -124,7 +117,7 @@ def profile_gemv(args):
     dev = "cuda:0"
     ws = L.GemvWorkspace(dev, floats=16 << 20)
     n, k = 51200, 5120
-    lins = [L.WqLinear.random(n, k, args.bits, 128, dev, seed=i, ks=args.ks or L.choose_ks(n, k)) for i in range(3)]
+    lins = [L.WqLinear.random(n, k, args.bits, 128, dev, seed=i) for i in range(3)]
     x = torch.randn(args.m, k, device=dev).to(torch.bfloat16)
     out = torch.empty(args.m, n, dtype=torch.bfloat16, device=dev)
     for _ in range(2):
@@ -379,7 +372,6 @@ def main(argv=None):
     ap.add_argument("what", choices=["gemv", "bf16", "attn", "gemm", "profile_gemv", "mm", "profile_mm", "profile_attn", "profile_attn_tc", "profile_gemm", "profile_misc", "profile_step"])
     ap.add_argument("--layers", type=int, default=0)
     ap.add_argument("--bits", type=int, default=4)
-    ap.add_argument("--ks", type=int, default=0)
     ap.add_argument("--m", type=int, default=1)
     ap.add_argument("--small", action="store_true")
     ap.add_argument("--rows", type=int, default=256)

@@ -68,8 +68,9 @@ PREFILL_TC_MIN_TOKENS = 64          # chunks from this size run the tcgen05 kern
 
 def attn_prefill_tc(q: torch.Tensor, kv_pool: torch.Tensor, block_table: torch.Tensor, seq: int, pos0: int, hq: int,
                     hkv: int, status: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Causal attention of a prefill chunk on the tcgen05 tensor cores (``csrc/kernels/sm100/attn_prefill_tc.cu``):
-    128-row query tiles (128 / group-size tokens x the heads of one KV group), S and the per-block output in TMEM."""
+    """Causal attention of a prefill chunk on the tcgen05 tensor cores (``csrc/kernels/sm100/attn_prefill_tc.cu``): one or
+    two 128-row query tiles per CTA (128 / group-size tokens x the heads of one KV group), scores, probabilities and the
+    output in TMEM."""
     lib = _lib.cuda_lib()
     if not getattr(lib, "_pf_tc_declared", False):
         vp, i = C.c_void_p, C.c_int

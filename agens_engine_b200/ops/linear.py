@@ -1,7 +1,8 @@
 """Quantised linears on the GPU: FM weight holder + GEMV launcher (decode / verify / small batch).
 
 Python here only assembles argument blocks; the arithmetic is in ``csrc/kernels/sm100/wq_gemv8.cu`` (one to eight rows, more
-in chunks of eight), ``wq_mm.cu`` (tensor-core GEMM) and ``wq_gemv.cu`` (the tensor-parallel push epilogue).
+in chunks of eight), ``wq_mm.cu`` (tensor-core GEMM) and ``wq_gemv.cu`` (the tensor-parallel push epilogue, and matrices
+beyond the schedule of the first).
 """
 from __future__ import annotations
 
@@ -25,16 +26,16 @@ def fm_bytes(n: int, k: int, bits: int, group: int) -> int:
 
 
 def choose_rb(n: int) -> int:
-    """Row blocks per warp item: 64-row items when the matrix has enough rows to keep every warp busy."""
+    """Row blocks per warp item of ``wq_gemv.cu``: 64-row items when the matrix has enough rows to keep every warp busy."""
     if os.environ.get("B200E_GEMV_RB"):
         return int(os.environ["B200E_GEMV_RB"])
     return 4 if n >= 16384 else 2
 
 
 def choose_ks(n: int, k: int, slice_k: int = 2560) -> int:
-    """Number of k slices of a linear: a function of the shape only (never of the token count), so per-row
+    """Number of k slices of a linear in ``wq_gemv.cu``: a function of the shape only (never of the token count), so per-row
     arithmetic stays batch invariant.  Slices of about ``slice_k`` inputs keep the staged activations small and give
-    the persistent GEMV thousands of (panel, slice) work items to balance over the SMs."""
+    the kernel thousands of (panel, slice) work items to balance over the SMs."""
     slice_k = int(os.environ.get("B200E_SLICE_K", slice_k))
     nu = k // 128
     want = max(1, round(k / slice_k))
@@ -227,10 +228,6 @@ class GemvWorkspace:
 
 
 MM_MIN_ROWS = int(os.environ.get("B200E_MM_MIN_ROWS", "9"))     # token rows from which the tcgen05 GEMM takes over
-# Measurement aids of the push-epilogue GEMV (wq_gemv.cu).  Only a library built with B200E_NVCC_DEFS=-DB2_MEASURE reads
-# these fields; the production kernels have the modes compiled out, so a stray environment variable cannot change results.
-TRACE_BUFFER = None      # int64 CUDA tensor [CTAs * 8 warps * 8] that receives the GEMV's phase stamps
-GEMV_DEBUG = int(os.environ.get("B200E_GEMV_DEBUG", "0"))
 
 
 def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_STORE,
@@ -240,7 +237,8 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
          amax_val: Optional[torch.Tensor] = None, amax_idx: Optional[torch.Tensor] = None, n_valid: Optional[int] = None,
          yf: Optional[torch.Tensor] = None, tp: Optional[_lib.TpPush] = None):
     """Launch one GEMV on the current stream.  ``x``: bf16 ``[m, k]`` (``h`` when ``pro == PRO_NORM``).  More than
-    ``MM_MIN_ROWS - 1`` rows go to the tensor-core GEMM (:func:`mm`), which takes the same arguments."""
+    ``MM_MIN_ROWS - 1`` rows go to the tensor-core GEMM (:func:`mm`), which takes the same arguments.  The packed weights are
+    read before the kernel that runs just before has finished; everything else may come from that kernel."""
     if isinstance(lin, Bf16Linear):
         if tp is not None:
             raise ValueError("bf16 linears are not sharded: tensor-parallel models quantise them at load")
@@ -291,7 +289,6 @@ def gemv(lin: WqLinear, x: torch.Tensor, ws: GemvWorkspace, *, epi: int = EPI_ST
     else:
         a.vworkers = lib.b2_wq_gemv_vworkers(lin.n, lin.k, lin.ks, a.rb)
         a.fmax = lib.b2_wq_gemv_fmax(lin.n, lin.k, lin.ks, a.rb)
-        a.debug, a.trace = GEMV_DEBUG, ptr(TRACE_BUFFER)
         if tp is not None:
             a.tp = tp
         need = lib.b2_wq_gemv_scratch_floats(lin.n, lin.k, lin.ks, a.rb, m)

@@ -5,7 +5,7 @@
 // kernels/m1/m1_model.cu:1875-1895).
 //
 // Persistent: one CTA per SM walks 128 x 256 tiles.  Warp 0 feeds a 4-stage shared-memory ring with TMA (cp.async.bulk.tensor, 128-byte
-// swizzle, every CTA loads its own tiles); one elected thread of warp 1 issues tcgen05.mma (M 128, N 256, K 16 per instruction, operands
+// swizzle, every CTA loads its own tiles); the first lane of warp 1 issues tcgen05.mma (M 128, N 256, K 16 per instruction, operands
 // read through shared-memory descriptors, accumulator = 256 TMEM columns, two of them in turn) and commits stage releases
 // and the "accumulator ready" arrivals to mbarriers; warps 2..5 read the accumulator back with tcgen05.ld (each warp owns
 // the 32 TMEM lanes its warp id modulo 4 selects), add the optional residual, convert and store, while the next tile is

@@ -1,6 +1,6 @@
 // Fragment-major (FM) weight layout of the mixed 2/3/4-bit linears: record geometry, shared-memory fragment loads, code
-// extraction for mma.m16n8k16 and the bounded mbarrier / bulk-copy helpers shared by the GEMV kernel (wq_gemv.cu) and
-// the persistent decode-step kernel (step_kernel.cu).
+// extraction for mma.m16n8k16 and the bounded mbarrier / bulk-copy helpers shared by the GEMV kernels (wq_gemv8.cu,
+// wq_gemv.cu), the mixed-bit GEMM (wq_mm.cu), the expansion to bf16 (wq_tools.cu) and the decode-step kernel (step_kernel.cu).
 #pragma once
 #include "common.cuh"
 

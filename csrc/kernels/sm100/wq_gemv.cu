@@ -1,4 +1,6 @@
-// Mixed 2/3/4-bit dequant GEMV for decode, verify and small batches (m <= 32 tokens), sm_100a.
+// Mixed 2/3/4-bit dequant GEMV of up to 32 token rows with the tensor-parallel push epilogue (EPI_TP_RESID), sm_100a.  Every
+// other linear runs on wq_gemv8.cu, except matrices beyond its schedule (b2_wq_gemv8_takes: k above 163840) or, in the
+// allocation-free entry point, beyond the built-in scratch: those come here with the other epilogues.
 //
 // Replaces the reference's KT/KF/W4H GEMV family (kernels/src/w4_gemv.cu:280-2937, kernels/src/w4h.cu:140-553)
 // with one kernel family over the fragment-major ("FM") weight layout:
@@ -68,13 +70,6 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
   const unsigned U = (unsigned)nitems * (unsigned)nb;          // host checks U * V < 2^32
   auto range_lo = [&](int v) -> unsigned { return ((unsigned)v * U) / (unsigned)V; };
 
-#ifdef B2_MEASURE   // measurement builds only (B200E_NVCC_DEFS=-DB2_MEASURE): phase stamps and the bandwidth-probe mode
-  unsigned long long* tr = a.trace ? a.trace + ((size_t)blockIdx.x * kGemvWarps + warp) * 8 : nullptr;
-#else
-  unsigned long long* tr = nullptr;
-#endif
-  auto stamp = [&](int i) { if (tr && lane == 0) tr[i] = globaltimer_ns(); };
-  stamp(0);
   if (lane == 0) {
 #pragma unroll
     for (int i = 0; i < NST; ++i) mbar_init(bars_u + i * 8, 1);
@@ -115,10 +110,8 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
     while (prod - cons < (unsigned)NST && issue_one()) { }
   }
   __syncwarp();
-  stamp(1);
   pdl_wait();
-  pdl_launch_dependents();
-  stamp(2);   // the next kernel may start prefetching its weights while this one runs
+  pdl_launch_dependents();   // the next kernel may start prefetching its weights while this one runs
 
   // ---- stage the activation slice of this CTA: fp16(x / c) and the per-group sums ----
   if (a.pro == PRO_NORM) {
@@ -185,10 +178,8 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
     }
   }
   __syncthreads();
-  stamp(3);
 
   bool failed = false;
-  bool first_wait = true;
   for (int vw = wfirst; vw < V && nb > 0 && !failed; vw += wstride) {
    unsigned u = range_lo(vw);
    const unsigned u_end = range_lo(vw + 1);
@@ -214,19 +205,7 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
         failed = true;
         break;
       }
-      if (first_wait) { stamp(4); first_wait = false; }
       const uint8_t* stg = ring + slot * R::STAGE;
-#ifdef B2_MEASURE
-      if (a.debug == 1) {   // measurement aid: stream the weights, skip the arithmetic
-        y[0][0][0] += (float)stg[lane];
-        __syncwarp();
-        ++cons;
-        if (lane == 0) {
-          while (prod - cons < (unsigned)NST && issue_one()) { }
-        }
-        continue;
-      }
-#endif
       WFrag<BITS, GROUP> cf[RB];
 #pragma unroll
       for (int r = 0; r < RB; ++r)
@@ -294,7 +273,6 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
     if (failed) break;
 
     // ---- item done: fragment layout -> RPL rows per lane (row = lane + 32 j) ----
-    stamp(5);
     const int item = cur;
     const int n0 = item * ROWS;
     __syncwarp();
@@ -485,7 +463,6 @@ __global__ void __launch_bounds__(kGemvThreads) wq_gemv_kernel(const WqGemvArgs 
     }
    }
   }
-  stamp(6);
   if (failed) {
     // Give copies still in flight a bounded chance to land before the CTA's shared memory is released.
     const uint64_t t0 = globaltimer_ns();

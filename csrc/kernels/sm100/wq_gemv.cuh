@@ -1,4 +1,4 @@
-// Argument block of the mixed-bit dequant GEMV family (wq_gemv.cu) and of its tensor-parallel variant.
+// Argument block of the mixed-bit dequant GEMV family: wq_gemv8.cu, and wq_gemv.cu with the tensor-parallel epilogue.
 #pragma once
 #include "common.cuh"
 
@@ -39,9 +39,9 @@ struct WqGemvArgs {
   const uint8_t* wq;     // FM blocks [n/32][k/128][2 x records | 2 x groups x 16 x (scale, zero)]
   int n, k, m;
   int bits, group;
-  int ks;                // k slices (a function of the linear's shape only)
-  int rb;                // row blocks per warp item: 2 (32 rows) or 4 (64 rows)
-  int vworkers, fmax;    // b2_wq_gemv_vworkers / b2_wq_gemv_fmax of (n, k, ks, rb)
+  int ks;                // wq_gemv.cu: k slices (a function of the linear's shape only)
+  int rb;                // wq_gemv.cu: row blocks per warp item: 2 (32 rows) or 4 (64 rows)
+  int vworkers, fmax;    // wq_gemv.cu: b2_wq_gemv_vworkers / b2_wq_gemv_fmax of (n, k, ks, rb)
   int pro;
   const bf16* x; long ldx;
   const float* ss_in; int ss_parts; int ss_ld;
@@ -52,11 +52,9 @@ struct WqGemvArgs {
   float* ss_out;
   float* yf;
   float* amax_val; int* amax_idx; int n_valid;   // EPI_ARGMAX: rows >= n_valid never win
-  float* scratch; unsigned* counters;   // split-k partials [item][ks][m][16*rb] and self-resetting panel counters
+  float* scratch; unsigned* counters;   // partial results (b2_wq_gemv*_scratch_floats) and self-resetting panel counters
   int* status;           // device status word (B2_ERR_TIMEOUT when a bounded wait ran out)
-  int debug;             // read by -DB2_MEASURE builds only: 1 = stream weights without arithmetic (bandwidth probe)
   TpPush tp;
-  unsigned long long* trace;   // read by -DB2_MEASURE builds only: [CTA][warp][8] globaltimer stamps of the kernel's phases
 };
 
 }  // namespace b2

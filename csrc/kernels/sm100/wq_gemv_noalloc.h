@@ -3,7 +3,7 @@
 // Who needs it: callers that must not (or cannot) allocate device memory at the moment they want a GEMV -- code that
 // runs while a memory-budget cap leaves no headroom, plug-ins that are handed a fixed set of buffers by their host
 // application, and hosts that forbid cudaMalloc on their hot path because it synchronises the device.  The regular
-// entry point (b2_wq_gemv) expects the caller to bring split-k scratch memory, work counters and a status word; this
+// entry point (b2_wq_gemv8) expects the caller to bring split-k scratch memory, work counters and a status word; this
 // one keeps them in a fixed array inside the library.
 #pragma once
 #include <cuda_runtime.h>
