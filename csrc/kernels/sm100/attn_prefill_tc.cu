@@ -3,9 +3,9 @@
 // The reference's prefill attention is a flash kernel on mma.sync tiles (kernels/m1/m1_attn.cu:120-410, 64-row query
 // tiles, K/V through cp.async).  Here a query tile is 128 rows = (128 / gq) consecutive tokens x the gq query heads of
 // one KV head (GQA: the heads of a group share every K/V byte), the native M of tcgen05.mma.  A CTA owns two tiles and
-// walks the sequence in blocks of 128 keys (one tile where that leaves every CTA an SM of its own).  Warps 0-3 / 4-7 are the softmax of tile 0 / 1 (thread = row), warp 8 issues
-// the MMAs, warp 9 fetches K and V by TMA (a 16-token page of one head is 16 contiguous rows of 256 bytes; the 128-byte
-// swizzle is the tensor map's).  Per tile and block:
+// walks the sequence in blocks of 128 keys (one tile where that leaves every CTA an SM of its own).  Warps 0-3 / 4-7 are
+// the softmax of tile 0 / 1 (thread = row), warp 8 issues the MMAs, warp 9 fetches K and V by TMA (a 16-token page of one
+// head is 16 contiguous rows of 256 bytes; the 128-byte swizzle is the tensor map's).  Per tile and block:
 //   S (128 x 128, fp32, TMEM)  = Q (smem) x K^T (smem, K-major)                        8 MMAs of k = 16
 //   P = exp2((S - m) scale)    bf16, written over S in TMEM (tcgen05.st), the A operand of
 //   O (128 x 128, fp32, TMEM) += P (TMEM) x V (smem, MN-major)                         8 MMAs of k = 16
@@ -13,15 +13,15 @@
 // scores' registers are free.  Exponents are taken against the running maximum itself: scaling only after it had grown by
 // 2^8 was 4 % faster, but leaves a row's heaviest probabilities anywhere in a binade instead of at its top, where bf16
 // rounds best, and 2048 rows after 6144 tokens were 2.35e-3 from 64 bits instead of 2.30e-3.  The tensor core works on one
-// tile while the other is in its softmax; S(j + 1) follows P V(j) of the same tile in issue order, so S may overwrite P, and a finished S
-// implies a finished O.
+// tile while the other is in its softmax; S(j + 1) follows P V(j) of the same tile in issue order, so S may overwrite P, and
+// a finished S implies a finished O.
 //
 // What bounds it: at long contexts the softmax's issue slots (some 4.5 instructions a score: 1150 cycles a block of two
 // tiles) beside 2048 cycles of MMA at the nominal rate, and the last wave of CTAs (one per SM); short ones the chain of
 // launch, first copies, one block and output, for which Q comes by asynchronous copies (4 us sooner than load by load) and
 // the first two blocks of K and V are under way before it is there.  The kernel before had one tile of 128 threads per CTA,
 // S and P through registers and shared memory, O in registers and the copies in the same threads.  64 q / 8 kv heads,
-// before -> now: 2048 rows after 6144 tokens 1050 -> 510 us (945 TFLOP/s), after 8000 1322 -> 568, from 0 181 -> 102; 256
+// before -> now: 2048 rows after 6144 tokens 1050 -> 500 us (960 TFLOP/s), after 8000 1322 -> 568, from 0 181 -> 102; 256
 // rows after 8000 256 -> 122, from 0 13.2 -> 10.9; 64 rows from 0 7.2 -> 7.4.
 // Every wait is bounded; expiry sets the status word and the CTA leaves through the normal exit (TMEM is released).
 #include <cuda.h>

@@ -1,6 +1,6 @@
 // Mixed 2/3/4-bit dequant GEMV for one to eight token rows (decode, small verify blocks), sm_100a; more rows run in
 // chunks of eight.  Same weight layout, arithmetic per group and epilogues as wq_gemv.cu, whose kernel stays for the
-// tensor-parallel push epilogue.
+// tensor-parallel push epilogue and for matrices beyond the schedule here (b2_wq_gemv8_takes).
 //
 // Work: the units (32-row panel, 128-k batch) of the matrix.  k is cut into equal slices of at most 5120 inputs, so that
 // a CTA's activations fit its shared memory at eight rows, and every slice has the same number of CTAs; CTA c of a slice
@@ -11,15 +11,15 @@
 // so a row's bits do not depend on the rows that travel with it.
 //
 // One CTA of 16 warps per SM at full registers.  (64 registers and half of the shared memory, so that the next linear's
-// CTAs could prefetch beside this one, measured slower: 747 against 471 us for four 32B layers and the head at one row --
-// the early CTAs keep the attention kernels between the linears off the SMs.)
+// CTAs could prefetch beside this one, measured slower: four 32B layers and the head at one row 747 us, 420 in this form
+// with its slices of k -- the early CTAs keep the attention kernels between the linears off the SMs.)
 //
 // What bounds it: large matrices the inner loop (the logic pipe takes two cycles an instruction and scheduler, some 110 of
 // them a unit, and 16 half-precision MMAs of 8) and, at 4 bits, DRAM; small ones the fixed 4 us of launch, staging and
 // hand-over.  The kernel of wq_gemv.cu staged every row of a CTA's slice and summed every row's parts one after the
 // other, and its shared memory left one CTA of eight warps per SM from five rows on.  4 bits, graph replays over weights
-// larger than L2, before -> now: one row gate_up 36 -> 27 us, lm_head 82 -> 68 (floor 63), down 25 -> 18, qkv 14.0 ->
-// 11.4, o 13.6 -> 10.6, 4096 x 1024 7.2 -> 3.8; eight rows gate_up 101 -> 34, lm_head 199 -> 76, down 191 -> 25, qkv
+// larger than L2, before -> now: one row gate_up 36 -> 28 us, lm_head 82 -> 72 (floor 63), down 25 -> 19, qkv 14.0 ->
+// 11.5, o 13.6 -> 10.7, 4096 x 1024 7.2 -> 3.9; eight rows gate_up 101 -> 35, lm_head 199 -> 78, down 191 -> 26, qkv
 // 64 -> 16, o 79 -> 15.
 #include "wq_frag.cuh"
 #include "wq_gemv.cuh"

@@ -24,8 +24,8 @@
 // rate) and, above 128 tokens, the epilogue of a tile, since only one such accumulator fits TMEM.  The earlier kernel wrote
 // fp16 tiles to shared memory from a register ring and cut k into equal slices (80 tiles x 2 slices = two waves of 148).
 // 4 bits, graph replays over weights larger than L2, before -> now: 16 tokens qkv 55 -> 21 us, o 49 -> 19, gate_up 105 ->
-// 54, down 94 -> 34, lm_head 303 -> 137; 256 tokens qkv 215 -> 46, o 211 -> 49, gate_up 222 -> 120 (1120 TFLOP/s), down
-// 268 -> 79, lm_head 655 -> 320 (1250 TFLOP/s).
+// 56, down 94 -> 37, lm_head 303 -> 141; 256 tokens qkv 215 -> 46, o 211 -> 48, gate_up 222 -> 120 (1120 TFLOP/s), down
+// 268 -> 79, lm_head 655 -> 327 (1220 TFLOP/s).
 #include <cuda.h>
 
 #include "common.cuh"
@@ -576,7 +576,9 @@ B2_API int b2_wq_mm(const WqMmArgs* args, const bf16* x, long ldx, const float* 
   const int raw = 8 * (a.bits == 3 ? 768 : (a.bits == 4 ? 1024 : 512)) + 8 * (128 / a.group) * 64;
   const int x_sub = a.n_pad * BKS * 2;
   // A step of two units halves the issuing warps' cost per unit; its three buffers take 384 TMEM columns, which leaves two
-  // accumulators of 64 tokens.
+  // accumulators of 64 tokens.  With four buffers a dequantiser set uses a buffer every third time only: that its wait for
+  // the commit of step st - 4 cannot take the phase of st - 8 for it rests on the commits of one thread arriving in order, of
+  // which it saw st - 7 a whole dequantisation earlier.  Three buffers there: 5120 x 25600 at 72 tokens 44 -> 48 us, else equal.
   a.per = a.n_pad <= 64 ? 2 : 1;
   a.bufs = a.n_pad <= 64 ? 3 : (a.n_pad <= 160 ? 4 : 3);
   const int left = 220 * 1024 - a.bufs * a.per * 2 * x_sub;
