@@ -220,11 +220,12 @@ class GemvWorkspace:
         return self.x16
 
     def ensure_scratch(self, floats: int):
-        """A larger linear than the workspace was sized for makes the scratch grow.  What it replaces is kept: CUDA graphs
-        captured before go on using that memory."""
-        if floats > self.scratch.numel():
+        """A larger linear than the workspace was sized for makes the scratch grow, by half at least.  What it replaces is
+        kept (twice the present size in all, at most): CUDA graphs captured before go on using that memory."""
+        have = self.scratch.numel()
+        if floats > have:
             self._outgrown.append(self.scratch)
-            self.scratch = torch.empty(floats, dtype=torch.float32, device=self.scratch.device)
+            self.scratch = torch.empty(max(floats, have + have // 2), dtype=torch.float32, device=self.scratch.device)
 
 
 MM_MIN_ROWS = int(os.environ.get("B200E_MM_MIN_ROWS", "9"))     # token rows from which the tcgen05 GEMM takes over

@@ -61,6 +61,19 @@ def test_allocation_free_gemv_near_its_limit(n, k, ks, m, bits):
     assert torch.equal(one[0], y[m - 1])
 
 
+def test_workspace_growth_is_bounded():
+    """Many small steps up: what is kept stays within twice the present size, and buffers handed out stay alive."""
+    from agens_engine_b200.ops import linear as L
+    ws = L.GemvWorkspace("cpu", floats=100, panels=4)
+    first = ws.scratch.data_ptr()
+    for n in range(100, 5000, 7):
+        ws.ensure_scratch(n)
+        assert ws.scratch.numel() >= n and sum(t.numel() for t in ws._outgrown) <= 2 * ws.scratch.numel()
+    assert ws._outgrown[0].data_ptr() == first and ws.scratch.numel() < 1.5 * 5000 + 1
+    ws.ensure_scratch(3)
+    assert ws.scratch.numel() >= 5000 - 7
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,k,floats", [(151936, 5248, 4 << 20), (2048, 5248, 1 << 10)])
 def test_gemv_grows_its_workspace(n, k, floats):
