@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) attn_prefill_tc_kernel(const __
             pf_mma_ts(tmem + 256u + (uint32_t)t * 128u, tmem + (uint32_t)t * 128u + (uint32_t)k * 8u,
                       pf_desc_mn(base + SM_V + st * 32768 + k * 2048, 16384, 1024), idesc_o, (j || k) ? 1u : 0u);
           if (j == nb - 1) pf_commit(smem_u32(&o_final[t]));
-          if (t == last) pf_commit(smem_u32(&v_empty[st]));
+          if (t == last && j + 2 < nb) pf_commit(smem_u32(&v_empty[st]));   // no arrival is left for after the last wait
           if (j + 1 < nb) {
             issue_s(t, sn);
             if (t == last) pf_commit(smem_u32(&k_empty[sn]));
